@@ -247,7 +247,7 @@ struct sf_world {
     std::vector<int32_t> h_sid;
     std::vector<uint32_t> h_s_cell;
     // bodies
-    sf::DBuf<float4> b_pos, b_q, b_v, b_w, b_vpre, b_wpre;
+    sf::DBuf<float4> b_pos, b_q, b_v, b_w;
     sf::DBuf<float> b_rot, b_iil, b_iiw, b_m, b_im, b_rad, b_sleep, b_maxr;
     sf::DBuf<uint8_t> b_alive, b_asleep, b_wake;
     sf::DBuf<uint32_t> b_first, b_count, b_nc, b_scene;

@@ -53,6 +53,10 @@ struct StepState {
     DBuf<uint32_t> mflag, mpos, pair_start, cflag, cpos;
     DBuf<uint32_t> man_a, man_b, man_start, man_count, man_prio, man_color, man_round;
     DBuf<float4> S_n, S_t1, S_t2, S_ra, S_rb, S_j;
+    DBuf<uint4> M_id;               // per manifold in colour-list order: its bodies and contact count,
+    DBuf<float4> M_k;               // and its bodies' inverse masses and inertias, five float4 columns
+    DBuf<float4> vw;                // per active-list body: velocity and spin as the solve moves them (b_v, b_w keep those
+                                    // before it)
     // contact reduction: per pair a big flag and its place among the big pairs, per big pair 27 best scores and 27
     // winners, per sorted contact a keep flag and its place among the kept
     DBuf<uint32_t> red_big, red_pos, red_keep, red_kpos, red_slots;
@@ -100,6 +104,7 @@ struct StepState {
     uint64_t capacity = 0;
     uint64_t last_contacts = 0;
     int solve_occ = 1, jp_occ = 1;
+    bool team_ok = false;        // the device can hold k_solve_team's cluster
     uint32_t max_scene_bodies = 0;
     // launch-shape tuning: pending timings of this step's tuned launches
     Tuner solve_t;
@@ -767,11 +772,14 @@ struct PrepArgs {
     float h;
     uint32_t nseg;                           // (domain, colour) segments of the colour lists
     const uint32_t *nm_p;                    // manifolds of the substep (device count)
-    const uint32_t *perm, *man_a, *man_b, *man_count;
+    const uint32_t *perm, *man_a, *man_b, *man_ca, *man_cb, *man_count;
     const uint32_t *man_start, *col_start, *col_list, *jds_off;
     const float4 *L_p, *L_n, *pos, *v, *w;
     const float *im, *iiw;
     float4 *S_n, *S_t1, *S_t2, *S_ra, *S_rb, *S_j;
+    uint4 *M_id;
+    float4 *M_k;
+    size_t m_cap;                            // manifolds a column of M_k holds
     uint32_t *invperm;
     // warm start: the last substep's table, read when `warm` is set
     int warm;
@@ -809,7 +817,16 @@ __global__ void k_prep(PrepArgs A) {
 #pragma unroll
         for (int q = 0; q < 9; q++) iib[q] = A.iiw[(size_t)b * 9 + q];
         imb = A.im[b];
+    } else {
+#pragma unroll
+        for (int q = 0; q < 9; q++) iib[q] = 0.0f;
     }
+    A.M_id[i] = make_uint4(A.man_ca[m], A.man_cb[m], cnt, 0u);
+    A.M_k[i] = make_float4(iia[0], iia[1], iia[2], iia[3]);
+    A.M_k[A.m_cap + i] = make_float4(iia[4], iia[5], iia[6], iia[7]);
+    A.M_k[2 * A.m_cap + i] = make_float4(iia[8], ima, iib[0], iib[1]);
+    A.M_k[3 * A.m_cap + i] = make_float4(iib[2], iib[3], iib[4], iib[5]);
+    A.M_k[4 * A.m_cap + i] = make_float4(iib[6], iib[7], iib[8], imb);
     const uint32_t *off = A.jds_off + c * JDS_K;
     for (uint32_t kk = 0; kk < cnt; kk++) {
         const uint32_t d = off[kk] + p;
@@ -1133,12 +1150,14 @@ struct SolveArgs {
     const uint4 *blk_dom;          // per block: domain, rank in the domain, blocks of the domain
     const uint32_t *dom_ncol;      // per domain: colours used
     uint32_t cstride;              // segment of (domain d, colour c) = d * cstride + c
-    const uint32_t *col_start, *col_list, *jds_off;
-    const uint32_t *man_a, *man_b, *man_count;
+    const uint32_t *col_start, *jds_off;
+    const uint4 *M_id;
+    const float4 *M_k;
+    size_t m_cap;
     const float4 *S_n, *S_t1, *S_t2, *S_ra, *S_rb;
     float4 *S_j;
-    float4 *v, *w;
-    const float *im, *iiw;
+    float4 *vw;                    // per active-list body: velocity, spin
+    uint32_t nb;                   // active-list bodies
     GridBarrier *gb;
     uint32_t *err;
     uint32_t warm;                 // 1: a first pass applies the warm-started impulses
@@ -1151,125 +1170,116 @@ template <bool ONE_BLOCK> __device__ __forceinline__ float4 ld_rw(const float4 *
     return __ldcg(p);
 }
 
-template <bool ONE_BLOCK>
-__device__ __forceinline__ void solve_manifold(const SolveArgs &A, uint32_t m, uint32_t p, const uint32_t *off) {
-    const uint32_t a = A.man_a[m], b = A.man_b[m];
-    const bool hasb = b != STATIC;
-    const uint32_t cnt = A.man_count[m];
-    float4 t4 = ld_rw<ONE_BLOCK>(&A.v[a]);
-    V3 va = v3(t4.x, t4.y, t4.z);
-    t4 = ld_rw<ONE_BLOCK>(&A.w[a]);
-    V3 wa = v3(t4.x, t4.y, t4.z);
-    const float ima = A.im[a];
-    float ia[9], ib[9];
-#pragma unroll
-    for (int q = 0; q < 9; q++) ia[q] = A.iiw[(size_t)a * 9 + q];
-    V3 vb = v3(0.0f, 0.0f, 0.0f), wb = v3(0.0f, 0.0f, 0.0f);
-    float imb = 0.0f;
-    if (hasb) {
-        t4 = ld_rw<ONE_BLOCK>(&A.v[b]); vb = v3(t4.x, t4.y, t4.z);
-        t4 = ld_rw<ONE_BLOCK>(&A.w[b]); wb = v3(t4.x, t4.y, t4.z);
-        imb = A.im[b];
-#pragma unroll
-        for (int q = 0; q < 9; q++) ib[q] = A.iiw[(size_t)b * 9 + q];
+// A manifold's bodies with their masses, read in colour-list order (prep writes them so): a warp's 32 manifolds then take
+// a few dozen wavefronts of coalesced columns instead of ten scattered words a body, which kept the load units busier
+// than the memory: 1,666 -> 1,405 us for 8 iterations of 3.67M contacts (1.12M manifolds, 9 colours).
+struct Pair {
+    uint32_t a, b, cnt;
+    bool hasb;
+    V3 va, wa, vb, wb;
+    float ima, imb, ia[9], ib[9];
+};
+__device__ __forceinline__ Pair load_pair(const SolveArgs &A, uint32_t i) {
+    Pair P;
+    const uint4 id = __ldg(&A.M_id[i]);
+    P.a = id.x; P.b = id.y; P.cnt = id.z;
+    const float4 k0 = __ldg(&A.M_k[i]), k1 = __ldg(&A.M_k[A.m_cap + i]), k2 = __ldg(&A.M_k[2 * A.m_cap + i]);
+    const float4 k3 = __ldg(&A.M_k[3 * A.m_cap + i]), k4 = __ldg(&A.M_k[4 * A.m_cap + i]);
+    P.ia[0] = k0.x; P.ia[1] = k0.y; P.ia[2] = k0.z; P.ia[3] = k0.w; P.ia[4] = k1.x; P.ia[5] = k1.y; P.ia[6] = k1.z; P.ia[7] = k1.w;
+    P.ia[8] = k2.x; P.ima = k2.y; P.ib[0] = k2.z; P.ib[1] = k2.w; P.ib[2] = k3.x; P.ib[3] = k3.y; P.ib[4] = k3.z; P.ib[5] = k3.w;
+    P.ib[6] = k4.x; P.ib[7] = k4.y; P.ib[8] = k4.z; P.imb = k4.w;
+    return P;
+}
+// the velocities, through L2 (other blocks move them)
+__device__ __forceinline__ void load_vel(const SolveArgs &A, Pair &P) {
+    const float4 va = __ldcg(&A.vw[2 * (size_t)P.a]), wa = __ldcg(&A.vw[2 * (size_t)P.a + 1]);
+    P.va = v3(va.x, va.y, va.z);
+    P.wa = v3(wa.x, wa.y, wa.z);
+    P.vb = v3(0.0f, 0.0f, 0.0f);
+    P.wb = P.vb;
+    P.hasb = P.b != STATIC;
+    if (P.hasb) {
+        const float4 vb = __ldcg(&A.vw[2 * (size_t)P.b]), wb = __ldcg(&A.vw[2 * (size_t)P.b + 1]);
+        P.vb = v3(vb.x, vb.y, vb.z);
+        P.wb = v3(wb.x, wb.y, wb.z);
     }
-    // the next contact's data is loaded while the current one is solved (the chain through the bodies is serial)
-    float4 nx_n = make_float4(0, 0, 0, 0), nx_t1 = nx_n, nx_t2 = nx_n, nx_ra = nx_n, nx_rb = nx_n, nx_j = nx_n;
-    uint32_t at = off[0] + p;
-    if (cnt) {
-        nx_n = __ldg(&A.S_n[at]); nx_t1 = __ldg(&A.S_t1[at]); nx_t2 = __ldg(&A.S_t2[at]);
-        nx_ra = __ldg(&A.S_ra[at]); nx_rb = __ldg(&A.S_rb[at]); nx_j = ld_rw<ONE_BLOCK>(&A.S_j[at]);
-    }
-    for (uint32_t k = 0; k < cnt; k++) {
-        const float4 n4 = nx_n, t14 = nx_t1, t24 = nx_t2, ra4 = nx_ra, rb4 = nx_rb;
-        float4 j4 = nx_j;
-        const uint32_t cur = at;
-        if (k + 1 < cnt) {
-            at = off[k + 1] + p;
-            nx_n = __ldg(&A.S_n[at]); nx_t1 = __ldg(&A.S_t1[at]); nx_t2 = __ldg(&A.S_t2[at]);
-            nx_ra = __ldg(&A.S_ra[at]); nx_rb = __ldg(&A.S_rb[at]); nx_j = ld_rw<ONE_BLOCK>(&A.S_j[at]);
-        }
-        const V3 n = v3(n4.x, n4.y, n4.z), t1 = v3(t14.x, t14.y, t14.z), t2 = v3(t24.x, t24.y, t24.z);
-        const V3 ra = v3(ra4.x, ra4.y, ra4.z), rb = v3(rb4.x, rb4.y, rb4.z);
-        const float mn = n4.w, mt1 = t14.w, mt2 = t24.w, bias = ra4.w;
-        // normal
-        V3 dv = sub(add(va, cross(wa, ra)), hasb ? add(vb, cross(wb, rb)) : v3(0.0f, 0.0f, 0.0f));
-        float vn = dot(dv, n);
-        float lam = mn * (-vn + bias);
-        float old = j4.x;
-        j4.x = maxf(old + lam, 0.0f);
-        float d = j4.x - old;
-        {
-            V3 P = mul(n, d);
-            va = madd(va, P, ima);
-            wa = add(wa, mv(ia, cross(ra, P)));
-            if (hasb) { vb = madd(vb, P, -imb); wb = sub(wb, mv(ib, cross(rb, P))); }
-        }
-        // friction, two independent clamps
-        float lim = MU * j4.x;
-        dv = sub(add(va, cross(wa, ra)), hasb ? add(vb, cross(wb, rb)) : v3(0.0f, 0.0f, 0.0f));
-        float l1 = -mt1 * dot(dv, t1);
-        float o1 = j4.y;
-        j4.y = clampf(o1 + l1, -lim, lim);
-        float l2 = -mt2 * dot(dv, t2);
-        float o2 = j4.z;
-        j4.z = clampf(o2 + l2, -lim, lim);
-        {
-            V3 P = add(mul(t1, j4.y - o1), mul(t2, j4.z - o2));
-            va = madd(va, P, ima);
-            wa = add(wa, mv(ia, cross(ra, P)));
-            if (hasb) { vb = madd(vb, P, -imb); wb = sub(wb, mv(ib, cross(rb, P))); }
-        }
-        A.S_j[cur] = j4;
-    }
-    A.v[a] = make_float4(va.x, va.y, va.z, 0.0f);
-    A.w[a] = make_float4(wa.x, wa.y, wa.z, 0.0f);
-    if (hasb) {
-        A.v[b] = make_float4(vb.x, vb.y, vb.z, 0.0f);
-        A.w[b] = make_float4(wb.x, wb.y, wb.z, 0.0f);
+}
+__device__ __forceinline__ void store_vel(const SolveArgs &A, const Pair &P) {
+    A.vw[2 * (size_t)P.a] = make_float4(P.va.x, P.va.y, P.va.z, 0.0f);
+    A.vw[2 * (size_t)P.a + 1] = make_float4(P.wa.x, P.wa.y, P.wa.z, 0.0f);
+    if (P.hasb) {
+        A.vw[2 * (size_t)P.b] = make_float4(P.vb.x, P.vb.y, P.vb.z, 0.0f);
+        A.vw[2 * (size_t)P.b + 1] = make_float4(P.wb.x, P.wb.y, P.wb.z, 0.0f);
     }
 }
 
-// the warm-started impulses of a manifold's contacts, applied once in its order (apply_imp with the whole impulse)
+struct Contact { float4 n, t1, t2, ra, rb, j; };   // n | mn, t1 | mt1, t2 | mt2, ra | bias, rb | vn0, impulses
 template <bool ONE_BLOCK>
-__device__ __forceinline__ void warm_manifold(const SolveArgs &A, uint32_t m, uint32_t p, const uint32_t *off) {
-    const uint32_t a = A.man_a[m], b = A.man_b[m];
-    const bool hasb = b != STATIC;
-    const uint32_t cnt = A.man_count[m];
-    float4 t4 = ld_rw<ONE_BLOCK>(&A.v[a]);
-    V3 va = v3(t4.x, t4.y, t4.z);
-    t4 = ld_rw<ONE_BLOCK>(&A.w[a]);
-    V3 wa = v3(t4.x, t4.y, t4.z);
-    const float ima = A.im[a];
-    float ia[9], ib[9];
-#pragma unroll
-    for (int q = 0; q < 9; q++) ia[q] = A.iiw[(size_t)a * 9 + q];
-    V3 vb = v3(0.0f, 0.0f, 0.0f), wb = v3(0.0f, 0.0f, 0.0f);
-    float imb = 0.0f;
-    if (hasb) {
-        t4 = ld_rw<ONE_BLOCK>(&A.v[b]); vb = v3(t4.x, t4.y, t4.z);
-        t4 = ld_rw<ONE_BLOCK>(&A.w[b]); wb = v3(t4.x, t4.y, t4.z);
-        imb = A.im[b];
-#pragma unroll
-        for (int q = 0; q < 9; q++) ib[q] = A.iiw[(size_t)b * 9 + q];
+__device__ __forceinline__ Contact load_contact(const SolveArgs &A, uint32_t at) {
+    Contact c;
+    c.n = __ldg(&A.S_n[at]); c.t1 = __ldg(&A.S_t1[at]); c.t2 = __ldg(&A.S_t2[at]);
+    c.ra = __ldg(&A.S_ra[at]); c.rb = __ldg(&A.S_rb[at]); c.j = ld_rw<ONE_BLOCK>(&A.S_j[at]);
+    return c;
+}
+// solve() of one contact (src/lib.rs:1579-1601); its new impulses are returned. STRAIGHT computes the second body's side
+// without branches also where there is none (zero mass and arms; its velocity at the contact is then replaced by 0), so
+// that the two sides' chains interleave: a lane of a small substep is alone on its scheduler.
+template <bool STRAIGHT>
+__device__ __forceinline__ float4 solve_contact(Pair &P, const Contact &c) {
+    const bool hasb = P.hasb;
+    float4 j4 = c.j;
+    const V3 n = v3(c.n.x, c.n.y, c.n.z), t1 = v3(c.t1.x, c.t1.y, c.t1.z), t2 = v3(c.t2.x, c.t2.y, c.t2.z);
+    const V3 ra = v3(c.ra.x, c.ra.y, c.ra.z), rb = v3(c.rb.x, c.rb.y, c.rb.z);
+    auto relative = [&]() {
+        const V3 a = add(P.va, cross(P.wa, ra));
+        if (!STRAIGHT) return sub(a, hasb ? add(P.vb, cross(P.wb, rb)) : v3(0.0f, 0.0f, 0.0f));
+        const V3 b = add(P.vb, cross(P.wb, rb));
+        return v3(a.x - (hasb ? b.x : 0.0f), a.y - (hasb ? b.y : 0.0f), a.z - (hasb ? b.z : 0.0f));
+    };
+    auto apply = [&](V3 I) {
+        P.va = madd(P.va, I, P.ima);
+        P.wa = add(P.wa, mv(P.ia, cross(ra, I)));
+        if (STRAIGHT || hasb) { P.vb = madd(P.vb, I, -P.imb); P.wb = sub(P.wb, mv(P.ib, cross(rb, I))); }
+    };
+    // (fmaxf is maxf here: its second operand wins on NaN, and where the two zeros differ the next minf or the sum hides it)
+    // normal
+    const float lam = c.n.w * (-dot(relative(), n) + c.ra.w);
+    const float old = j4.x;
+    j4.x = fmaxf(old + lam, 0.0f);
+    apply(mul(n, j4.x - old));
+    // friction, two independent clamps
+    const float lim = MU * j4.x;
+    const V3 dv = relative();
+    const float l1 = -c.t1.w * dot(dv, t1), o1 = j4.y;
+    j4.y = minf(fmaxf(o1 + l1, -lim), lim);
+    const float l2 = -c.t2.w * dot(dv, t2), o2 = j4.z;
+    j4.z = minf(fmaxf(o2 + l2, -lim), lim);
+    apply(add(mul(t1, j4.y - o1), mul(t2, j4.z - o2)));
+    return j4;
+}
+// the warm-started impulses of a contact, applied once (apply_imp with the whole impulse)
+__device__ __forceinline__ void warm_contact(Pair &P, const Contact &c) {
+    const V3 ra = v3(c.ra.x, c.ra.y, c.ra.z), rb = v3(c.rb.x, c.rb.y, c.rb.z);
+    const V3 I = add(mul(v3(c.n.x, c.n.y, c.n.z), c.j.x),
+                     add(mul(v3(c.t1.x, c.t1.y, c.t1.z), c.j.y), mul(v3(c.t2.x, c.t2.y, c.t2.z), c.j.z)));
+    P.va = madd(P.va, I, P.ima);
+    P.wa = add(P.wa, mv(P.ia, cross(ra, I)));
+    if (P.hasb) { P.vb = madd(P.vb, I, -P.imb); P.wb = sub(P.wb, mv(P.ib, cross(rb, I))); }
+}
+
+// manifold i of the colour lists, the p-th of its colour
+__device__ __forceinline__ void solve_manifold(const SolveArgs &A, uint32_t i, uint32_t p, const uint32_t *off, bool warm) {
+    Pair P = load_pair(A, i);
+    load_vel(A, P);
+    // the next contact's data is loaded while the current one is solved (the chain through the bodies is serial)
+    Contact nx = load_contact<false>(A, off[0] + p);
+    for (uint32_t k = 0; k < P.cnt; k++) {
+        const Contact c = nx;
+        if (k + 1 < P.cnt) nx = load_contact<false>(A, off[k + 1] + p);
+        if (warm) warm_contact(P, c);
+        else A.S_j[off[k] + p] = solve_contact<false>(P, c);
     }
-    for (uint32_t k = 0; k < cnt; k++) {
-        const uint32_t at = off[k] + p;
-        const float4 n4 = __ldg(&A.S_n[at]), t14 = __ldg(&A.S_t1[at]), t24 = __ldg(&A.S_t2[at]);
-        const float4 ra4 = __ldg(&A.S_ra[at]), rb4 = __ldg(&A.S_rb[at]), j4 = ld_rw<ONE_BLOCK>(&A.S_j[at]);
-        const V3 ra = v3(ra4.x, ra4.y, ra4.z), rb = v3(rb4.x, rb4.y, rb4.z);
-        const V3 P = add(mul(v3(n4.x, n4.y, n4.z), j4.x),
-                         add(mul(v3(t14.x, t14.y, t14.z), j4.y), mul(v3(t24.x, t24.y, t24.z), j4.z)));
-        va = madd(va, P, ima);
-        wa = add(wa, mv(ia, cross(ra, P)));
-        if (hasb) { vb = madd(vb, P, -imb); wb = sub(wb, mv(ib, cross(rb, P))); }
-    }
-    A.v[a] = make_float4(va.x, va.y, va.z, 0.0f);
-    A.w[a] = make_float4(wa.x, wa.y, wa.z, 0.0f);
-    if (hasb) {
-        A.v[b] = make_float4(vb.x, vb.y, vb.z, 0.0f);
-        A.w[b] = make_float4(wb.x, wb.y, wb.z, 0.0f);
-    }
+    store_vel(A, P);
 }
 
 constexpr int SOLVE_BLOCK = 128;
@@ -1299,38 +1309,183 @@ __global__ void __launch_bounds__(SOLVE_BLOCK) k_solve(SolveArgs A) {
             const uint32_t s0 = A.col_start[seg], n = A.col_start[seg + 1] - s0;
             for (uint32_t r = 0; r * stride < n; r++) {
                 const uint32_t p = snake_pos(r, g, stride);
-                if (p < n) {
-                    if (wp) warm_manifold<false>(A, A.col_list[s0 + p], p, off);
-                    else solve_manifold<false>(A, A.col_list[s0 + p], p, off);
-                }
+                if (p < n) solve_manifold(A, s0 + p, p, off, wp);
             }
             if (!dom_sync(A.gb + d, nblk, A.err)) return;
         }
     }
 }
 
-// small substeps: one block, colours separated by __syncthreads instead of a grid barrier
-constexpr int SOLVE_ONE_BLOCK = 512;
-constexpr uint32_t SOLVE_ONE_BLOCK_MAX_CONTACTS = 8192;
-constexpr uint32_t SMALL_SUBSTEP_CONTACTS = 1024;
-__global__ void __launch_bounds__(SOLVE_ONE_BLOCK) k_solve_one_block(SolveArgs A) {
-    __shared__ uint32_t off[JDS_K];
-    const uint32_t ncol = A.dev[DV_COLORS];
-    for (uint32_t it = 0; it < A.iterations + A.warm; it++) {
-        const bool wp = A.warm && it == 0;
-        for (uint32_t c = 0; c < ncol; c++) {
-            if (threadIdx.x < JDS_K) off[threadIdx.x] = A.jds_off[c * JDS_K + threadIdx.x];
+// Small substeps (at most SOLVE_TEAM_MAX contacts): one block (NB = 1), or one cluster of NB blocks, with everything the
+// iterations touch in shared memory: the active bodies' velocities (body t in block t % NB) and the contacts (position p
+// of a colour in block p % NB). What bounds a colour pass there is the chain of its longest manifold, up to 32 contacts of
+// some 300 dependent-issue operations; read from L2 a contact took 780 to 930 cycles, the latency of its six words.
+// Solve of 8 iterations, against one block (or warp) that read everything through L1: 1,300 contacts 140 -> 107 us (alone;
+// 114 on the cluster), 2,980 198 -> 143 us, 3,600 242 -> 133 us, 7,580 288 -> 147 us. A contact now takes 590 cycles, about
+// its instructions at one every two cycles of the one warp that runs the chain.
+constexpr int SOLVE_TEAM_BLOCKS = 16, SOLVE_TEAM_T = 128, SOLVE_TEAM_T1 = 256;   // threads a block of the cluster / alone
+constexpr uint32_t SOLVE_TEAM_MAX = 8192;          // contacts
+constexpr uint32_t SMALL_SUBSTEP_CONTACTS = 1024;  // contacts up to which the colouring runs on one block
+constexpr uint32_t SOLVE_TEAM_COLS = 64;           // colours whose tables are kept in shared memory
+constexpr uint32_t SOLVE_TEAM_SMEM = 196 * 1024;
+constexpr uint32_t SOLVE_TEAM_BODIES = 4096;       // bodies a block
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_cluster_v3(uint32_t a, V3 v) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(0.0f) : "memory");
+}
+__device__ __forceinline__ void cp_async16(float4 *to, const float4 *from) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from) : "memory");
+}
+template <int NB, int T>
+__global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, uint32_t nc, uint32_t slots) {
+    extern __shared__ float4 sv[];                 // velocity, spin of bodies rank, rank + NB, ...; then the contacts
+    __shared__ uint32_t s_start[SOLVE_TEAM_COLS + 1], s_off[SOLVE_TEAM_COLS * JDS_K + 1], s_loc[SOLVE_TEAM_COLS * JDS_K + 1];
+    __shared__ uint32_t s_base[NB];                // shared::cluster address of every block's velocities
+    __shared__ uint32_t s_sum[T / 32];
+    const uint32_t rank = blockIdx.x, g = threadIdx.x * NB + rank, lane = threadIdx.x & 31;
+    constexpr uint32_t stride = NB * T;
+    const uint32_t ncol = A.dev[DV_COLORS], rows = ncol * JDS_K;
+    const bool tab = ncol <= SOLVE_TEAM_COLS;
+    const uint32_t nbl = (A.nb + NB - 1) / NB;
+    float4 *sc = sv + 2 * nbl;                     // six columns of `slots` contacts
+    uint32_t used = 0;
+    if (tab) {
+        for (uint32_t k = threadIdx.x; k <= ncol; k += T) s_start[k] = A.col_start[k];
+        for (uint32_t k = threadIdx.x; k <= rows; k += T) s_off[k] = k < rows ? A.jds_off[k] : nc;
+        __syncthreads();
+        // row (colour, k): the k-th contacts of the colour's manifolds, n of them; those of this block are positions
+        // rank, rank + NB, ... and go to consecutive slots
+        for (uint32_t r0 = 0; r0 < rows; r0 += T) {
+            const uint32_t r = r0 + threadIdx.x, n = r < rows ? s_off[r + 1] - s_off[r] : 0u;
+            const uint32_t m = n > rank ? (n - rank + NB - 1) / NB : 0u;
+            uint32_t x = m;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= (uint32_t)o) x += y; }
+            if (lane == 31) s_sum[threadIdx.x >> 5] = x;
             __syncthreads();
-            const uint32_t s0 = A.col_start[c], n = A.col_start[c + 1] - s0;
-            for (uint32_t r = 0; r * blockDim.x < n; r++) {
-                const uint32_t p = snake_pos(r, threadIdx.x, blockDim.x);
-                if (p < n) {
-                    if (wp) warm_manifold<true>(A, A.col_list[s0 + p], p, off);
-                    else solve_manifold<true>(A, A.col_list[s0 + p], p, off);
-                }
-            }
+            uint32_t before = used, all = 0;
+            for (uint32_t w = 0; w < T / 32; w++) { if (w < threadIdx.x >> 5) before += s_sum[w]; all += s_sum[w]; }
+            if (r < rows) s_loc[r] = before + x - m;
+            used += all;
             __syncthreads();
         }
+        if (threadIdx.x == 0) s_loc[rows] = used;
+        __syncthreads();
+    }
+    const bool resident = tab && used <= slots;    // else the contacts are read from memory
+    const uint32_t *start = tab ? s_start : A.col_start, *offs = tab ? s_off : A.jds_off;
+    // the slots, in runs of one row: thread by thread over all of them
+    auto each_slot = [&](auto &&f) {
+        uint32_t r = 0;
+        for (uint32_t q = threadIdx.x; q < used; q += T) {
+            while (s_loc[r + 1] <= q) r++;
+            f(q, (size_t)s_off[r] + rank + (q - s_loc[r]) * NB);
+        }
+    };
+    if (resident)
+        each_slot([&](uint32_t q, size_t at) {
+            cp_async16(&sc[q], &A.S_n[at]);
+            cp_async16(&sc[slots + q], &A.S_t1[at]);
+            cp_async16(&sc[2 * slots + q], &A.S_t2[at]);
+            cp_async16(&sc[3 * slots + q], &A.S_ra[at]);
+            cp_async16(&sc[4 * slots + q], &A.S_rb[at]);
+            cp_async16(&sc[5 * slots + q], &A.S_j[at]);
+        });
+    for (uint32_t k = threadIdx.x; k * NB + rank < A.nb; k += T) {
+        const size_t t = (size_t)k * NB + rank;
+        cp_async16(&sv[2 * k], &A.vw[2 * t]);
+        cp_async16(&sv[2 * k + 1], &A.vw[2 * t + 1]);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (threadIdx.x < NB) {
+        const uint32_t own = (uint32_t)__cvta_generic_to_shared(sv);
+        uint32_t far = own;
+        if (NB != 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(own), "r"(threadIdx.x));
+        s_base[threadIdx.x] = far;
+    }
+    __syncthreads();
+    auto sync = [&]() {
+        if (NB == 1) __syncthreads();
+        else asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+    };
+    sync();
+    auto load_v = [&](uint32_t t, V3 &v, V3 &w) {
+        float4 a, b;
+        if (NB == 1) { a = sv[2 * t]; b = sv[2 * t + 1]; }
+        else { const uint32_t at = s_base[t % NB] + (t / NB) * 32u; a = ld_cluster_f4(at); b = ld_cluster_f4(at + 16); }
+        v = v3(a.x, a.y, a.z);
+        w = v3(b.x, b.y, b.z);
+    };
+    auto store_v = [&](uint32_t t, V3 v, V3 w) {
+        if (NB == 1) { sv[2 * t] = make_float4(v.x, v.y, v.z, 0.0f); sv[2 * t + 1] = make_float4(w.x, w.y, w.z, 0.0f); }
+        else { const uint32_t at = s_base[t % NB] + (t / NB) * 32u; st_cluster_v3(at, v); st_cluster_v3(at + 16, w); }
+    };
+    // this thread's manifolds: for each iteration and colour, the positions g, g + stride, ...; the next one's bodies and
+    // masses are loaded while the current one is solved
+    uint32_t c = 0, p = g, it = 0;
+    const uint32_t iters = ncol ? A.iterations + A.warm : 0u;
+    Pair nx;
+    auto prefetch = [&]() {
+        nx.cnt = 0;
+        if (it < iters && p < start[c + 1] - start[c]) nx = load_pair(A, start[c] + p);
+    };
+    prefetch();
+    while (it < iters) {
+        const uint32_t c0 = c, p0 = p;
+        const bool warm = A.warm && it == 0;
+        const bool last = p - g + stride >= start[c + 1] - start[c];   // the colour's last round
+        p += stride;
+        if (last) {
+            p = g;
+            if (++c == ncol) { c = 0; it++; }
+        }
+        Pair P = nx;
+        P.hasb = P.b != STATIC;
+        P.vb = P.wb = v3(0.0f, 0.0f, 0.0f);
+        if (P.cnt) {
+            load_v(P.a, P.va, P.wa);
+            if (P.hasb) load_v(P.b, P.vb, P.wb);
+        }
+        prefetch();
+        if (P.cnt) {
+            const uint32_t *off = offs + c0 * JDS_K;
+            if (resident) {
+                const uint32_t *loc = s_loc + c0 * JDS_K, lp = p0 / NB;
+                auto get = [&](uint32_t q) {
+                    Contact x;
+                    x.n = sc[q]; x.t1 = sc[slots + q]; x.t2 = sc[2 * slots + q]; x.ra = sc[3 * slots + q]; x.rb = sc[4 * slots + q];
+                    x.j = sc[5 * slots + q];
+                    return x;
+                };
+                Contact y = get(loc[0] + lp);
+                for (uint32_t k = 0; k < P.cnt; k++) {
+                    const Contact x = y;
+                    if (k + 1 < P.cnt) y = get(loc[k + 1] + lp);
+                    if (warm) warm_contact(P, x);
+                    else sc[5 * slots + loc[k] + lp] = solve_contact<true>(P, x);
+                }
+            } else {
+                for (uint32_t k = 0; k < P.cnt; k++) {
+                    const Contact x = load_contact<true>(A, off[k] + p0);
+                    if (warm) warm_contact(P, x);
+                    else A.S_j[off[k] + p0] = solve_contact<true>(P, x);
+                }
+            }
+            store_v(P.a, P.va, P.wa);
+            if (P.hasb) store_v(P.b, P.vb, P.wb);
+        }
+        if (last) sync();
+    }
+    sync();
+    if (resident) each_slot([&](uint32_t q, size_t at) { A.S_j[at] = sc[5 * slots + q]; });
+    for (uint32_t k = threadIdx.x; k * NB + rank < A.nb; k += T) {
+        const size_t t = (size_t)k * NB + rank;
+        A.vw[2 * t] = sv[2 * k];
+        A.vw[2 * t + 1] = sv[2 * k + 1];
     }
 }
 
@@ -1376,7 +1531,7 @@ struct IntArgs {
     int phase;   // 0: pinch clamps then integration; 1: the pinch clamps only; 2: integration only
     uint8_t *alive, *asleep;
     float4 *pos, *q, *v, *w;
-    const float4 *vpre, *wpre;
+    const float4 *vw;            // velocity and spin after the solve (v, w: before it)
     const float *rad;
     float *sleep;
     const float *maxr;
@@ -1398,10 +1553,11 @@ __global__ void k_integrate(IntArgs A) {
     const float rad = A.rad[b];
     // pinch_check (src/lib.rs:1746-1768)
     if (A.phase != 2) {
-        float4 p4 = A.wpre[b];
-        V3 wpre = v3(p4.x, p4.y, p4.z);
-        p4 = A.vpre[b];
-        V3 vpre = v3(p4.x, p4.y, p4.z);
+        const V3 vpre = v, wpre = w;
+        t4 = A.vw[2 * (size_t)t];
+        v = v3(t4.x, t4.y, t4.z);
+        t4 = A.vw[2 * (size_t)t + 1];
+        w = v3(t4.x, t4.y, t4.z);
         V3 dw = sub(w, wpre);
         float tip = len(dw) * rad;
         if (tip > 6.0f) w = madd(wpre, dw, div_rn(6.0f, tip));
@@ -1410,6 +1566,7 @@ __global__ void k_integrate(IntArgs A) {
         if (m >= 8.0f && A.kmat[A.first[b]] < SLUG) {
             if (A.pinch_kill && A.count[b] <= 6) {
                 A.alive[b] = 0;
+                A.v[b] = make_float4(v.x, v.y, v.z, 0.0f);
                 A.w[b] = make_float4(w.x, w.y, w.z, 0.0f);
                 return;
             }
@@ -1500,14 +1657,15 @@ __global__ void k_wake(uint32_t nb, const uint32_t *list, uint8_t *wake, const u
     wake[b] = 0;
     if (alive[b]) { asleep[b] = 0; sleep[b] = 0.0f; }
 }
-__global__ void k_save_pre(uint32_t nb, const uint32_t *list, const uint8_t *alive, const float4 *v, const float4 *w,
-                           float4 *vpre, float4 *wpre) {
+// the velocities the solve works on
+__global__ void k_solve_vel(uint32_t nb, const uint32_t *list, const uint8_t *alive, const float4 *v, const float4 *w,
+                            float4 *vw) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nb) return;
     const uint32_t b = pick(list, t);
     if (!alive[b]) return;
-    vpre[b] = v[b];
-    wpre[b] = w[b];
+    vw[2 * (size_t)t] = v[b];
+    vw[2 * (size_t)t + 1] = w[b];
 }
 __global__ void k_count_bodies(uint32_t nb, const uint8_t *alive, const uint8_t *asleep, uint32_t *dev) {
     uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1710,6 +1868,7 @@ sf_status step_create(sf_world *w) {
         SF_CUDA(S->dom_cnt.alloc(3 * DOM_MAX)); SF_CUDA(S->dom_gb.alloc(DOM_MAX));
     }
     if (w->P.manifold_chunk == 0 || w->P.manifold_chunk > (uint32_t)JDS_K) w->P.manifold_chunk = JDS_K;
+    SF_CUDA(S->vw.alloc(2 * (size_t)nb));
     SF_CUDA(S->parent.alloc(nb)); SF_CUDA(S->label.alloc(nb)); SF_CUDA(S->mint.alloc(nb));
     SF_CUDA(cudaMemsetAsync(S->label.p, 0xFF, S->label.bytes(), s));
     SF_CUDA(S->act_body.alloc(nb)); SF_CUDA(S->cidx.alloc(nb)); SF_CUDA(S->act_brick.alloc(nd));
@@ -1730,6 +1889,25 @@ sf_status step_create(sf_world *w) {
     uint64_t initial = w->P.contact_capacity ? w->P.contact_capacity : (uint64_t)std::max<uint32_t>(nd, 1) * 4;
     SF_CUDA(grow_contacts(S, initial));
     int occ = 0;
+    {
+        auto *one = k_solve_team<1, SOLVE_TEAM_T1>;
+        auto *team = k_solve_team<SOLVE_TEAM_BLOCKS, SOLVE_TEAM_T>;
+        SF_CUDA(cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLVE_TEAM_SMEM));
+        SF_CUDA(cudaFuncSetAttribute(team, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLVE_TEAM_SMEM));
+        SF_CUDA(cudaFuncSetAttribute(team, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchConfig_t c = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = SOLVE_TEAM_BLOCKS; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        c.gridDim = dim3(SOLVE_TEAM_BLOCKS);
+        c.blockDim = dim3(SOLVE_TEAM_T);
+        c.dynamicSmemBytes = SOLVE_TEAM_SMEM;
+        c.attrs = at;
+        c.numAttrs = 1;
+        int nc = 0;
+        if (cudaOccupancyMaxActiveClusters(&nc, team, &c) != cudaSuccess) { nc = 0; cudaGetLastError(); }
+        S->team_ok = nc > 0;
+    }
     SF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_solve, SOLVE_BLOCK, 0));
     S->solve_occ = std::max(1, occ);
     SF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_jp, SOLVE_BLOCK, 0));
@@ -1982,8 +2160,8 @@ static sf_status substep(sf_world *w, float h) {
     if (S->profile) S->sub_nc.push_back(nc);
     prof_mark(w);
     // The launch size of the colouring and the solve, and its partition into sync domains. A substep with few contacts
-    // is solved by one block (k_solve_one_block); its colouring then runs as a single domain.
-    const bool one_block = nc <= SOLVE_ONE_BLOCK_MAX_CONTACTS;
+    // is solved by one block or cluster (k_solve_team); its colouring then runs as a single domain.
+    const bool one_block = nc <= SOLVE_TEAM_MAX && nb <= (S->team_ok ? SOLVE_TEAM_BLOCKS : 1) * SOLVE_TEAM_BODIES;
     int sci = -1;
     const int sb = Tuner::bucket(nc);
     const unsigned top_occ = (unsigned)std::min(S->solve_occ, S->jp_occ);
@@ -2110,13 +2288,19 @@ static sf_status substep(sf_world *w, float h) {
             L++;
         }
         prof_mark(w);
+        // the solve's records are sized by the manifolds that occur (at most a contact each), not by the contact capacity
+        if (S->M_id.n < ncm) {
+            const size_t want = std::min<size_t>(S->capacity, 2 * (size_t)ncm + 65536);
+            SF_CUDA(S->M_id.alloc(want)); SF_CUDA(S->M_k.alloc(5 * want));
+        }
         PrepArgs PA;
         PA.nc = nc; PA.h = h; PA.nseg = nseg; PA.nm_p = S->dev.p + DV_MANIFOLDS; PA.perm = S->perm.p;
-        PA.man_a = S->man_a.p; PA.man_b = S->man_b.p; PA.man_count = S->man_count.p; PA.L_p = S->L_p.p; PA.L_n = S->L_n.p;
+        PA.man_a = S->man_a.p; PA.man_b = S->man_b.p; PA.man_ca = S->man_ca.p; PA.man_cb = S->man_cb.p; PA.man_count = S->man_count.p; PA.L_p = S->L_p.p; PA.L_n = S->L_n.p;
         PA.man_start = S->man_start.p; PA.col_start = S->col_start.p; PA.col_list = S->col_list.p;
         PA.jds_off = S->jds_off.p;
         PA.pos = w->b_pos.p; PA.v = w->b_v.p; PA.w = w->b_w.p; PA.im = w->b_im.p; PA.iiw = w->b_iiw.p;
         PA.S_n = S->S_n.p; PA.S_t1 = S->S_t1.p; PA.S_t2 = S->S_t2.p; PA.S_ra = S->S_ra.p; PA.S_rb = S->S_rb.p; PA.S_j = S->S_j.p;
+        PA.M_id = S->M_id.p; PA.M_k = S->M_k.p; PA.m_cap = S->M_id.n;
         PA.invperm = S->invperm.p;
         const bool warm_read = w->P.warm_start && S->warm_valid;
         const StepState::WarmTable &WT = S->warm[S->warm_cur];
@@ -2137,20 +2321,39 @@ static sf_status substep(sf_world *w, float h) {
         prof_mark(w);
         prof_mark(w);
     }
-    k_save_pre<<<grid_for(nb, 256), 256, 0, s>>>(nb, blist, w->b_alive.p, w->b_v.p, w->b_w.p, w->b_vpre.p, w->b_wpre.p);
+    k_solve_vel<<<grid_for(nb, 256), 256, 0, s>>>(nb, blist, w->b_alive.p, w->b_v.p, w->b_w.p, S->vw.p);
     L++;
     prof_mark(w);
     if (nc && w->P.iterations) {
         SolveArgs A;
-        A.iterations = w->P.iterations; A.dev = S->dev.p; A.col_start = S->col_start.p; A.col_list = S->col_list.p;
+        A.iterations = w->P.iterations; A.dev = S->dev.p; A.col_start = S->col_start.p;
         A.blk_dom = S->blk_dom.p; A.dom_ncol = S->dom_ncol.p; A.cstride = cstride;
-        A.jds_off = S->jds_off.p; A.man_a = S->man_a.p; A.man_b = S->man_b.p; A.man_count = S->man_count.p;
+        A.jds_off = S->jds_off.p; A.M_id = S->M_id.p; A.M_k = S->M_k.p; A.m_cap = S->M_id.n;
         A.S_n = S->S_n.p; A.S_t1 = S->S_t1.p; A.S_t2 = S->S_t2.p; A.S_ra = S->S_ra.p; A.S_rb = S->S_rb.p; A.S_j = S->S_j.p;
-        A.v = w->b_v.p; A.w = w->b_w.p; A.im = w->b_im.p; A.iiw = w->b_iiw.p; A.gb = S->dom_gb.p; A.err = w->err.p;
+        A.vw = S->vw.p; A.nb = nb; A.gb = S->dom_gb.p; A.err = w->err.p;
         A.warm = w->P.warm_start ? 1u : 0u;
         if (one_block) {
-            // a small substep's colours are short: one warp's barrier is cheaper than 16 warps'
-            k_solve_one_block<<<1, nc <= SMALL_SUBSTEP_CONTACTS / 2 ? 32 : SOLVE_ONE_BLOCK, 0, s>>>(A);
+            // alone a block holds the contacts of about 1,500 (SOLVE_TEAM_SMEM, 96 bytes each beside its bodies)
+            const bool alone = !S->team_ok || (uint64_t)nb * 32 + (uint64_t)ncm * 96 <= SOLVE_TEAM_SMEM;
+            const uint32_t nbl = alone ? nb : (nb + SOLVE_TEAM_BLOCKS - 1) / SOLVE_TEAM_BLOCKS;
+            // a block's contacts: an even share of each row (colour, k), rounded up
+            const uint32_t want = alone ? ncm : ncm / SOLVE_TEAM_BLOCKS + SOLVE_TEAM_COLS * JDS_K;
+            const uint32_t slots = std::min(want, (SOLVE_TEAM_SMEM - nbl * 32) / 96);
+            const size_t smem = (size_t)nbl * 32 + (size_t)slots * 96;
+            if (alone) k_solve_team<1, SOLVE_TEAM_T1><<<1, SOLVE_TEAM_T1, smem, s>>>(A, ncm, slots);
+            else {
+                cudaLaunchConfig_t cfg = {};
+                cudaLaunchAttribute at[1];
+                at[0].id = cudaLaunchAttributeClusterDimension;
+                at[0].val.clusterDim.x = SOLVE_TEAM_BLOCKS; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+                cfg.gridDim = dim3(SOLVE_TEAM_BLOCKS);
+                cfg.blockDim = dim3(SOLVE_TEAM_T);
+                cfg.dynamicSmemBytes = smem;
+                cfg.stream = s;
+                cfg.attrs = at;
+                cfg.numAttrs = 1;
+                SF_CUDA(cudaLaunchKernelEx(&cfg, k_solve_team<SOLVE_TEAM_BLOCKS, SOLVE_TEAM_T>, A, ncm, slots));
+            }
         } else {
             SF_CUDA(cudaMemsetAsync(S->dom_gb.p, 0, (size_t)S->part_D * sizeof(GridBarrier), s));
             void *sargs[] = {&A};
@@ -2195,7 +2398,7 @@ static sf_status substep(sf_world *w, float h) {
     IntArgs I;
     I.nb = nb; I.list = blist; I.h = h; I.pinch_kill = w->P.pinch_kill ? 1 : 0; I.island_mode = w->P.sleep_mode == SF_SLEEP_ISLAND;
     I.alive = w->b_alive.p; I.asleep = w->b_asleep.p; I.pos = w->b_pos.p; I.q = w->b_q.p; I.v = w->b_v.p; I.w = w->b_w.p;
-    I.vpre = w->b_vpre.p; I.wpre = w->b_wpre.p; I.rad = w->b_rad.p; I.sleep = w->b_sleep.p; I.maxr = w->b_maxr.p;
+    I.vw = S->vw.p; I.rad = w->b_rad.p; I.sleep = w->b_sleep.p; I.maxr = w->b_maxr.p;
     I.nc = w->b_nc.p; I.count = w->b_count.p; I.first = w->b_first.p; I.kmat = w->k_mat.p;
     I.phase = 0;
     if (w->P.damage && nc) {

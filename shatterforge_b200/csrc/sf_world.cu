@@ -641,7 +641,6 @@ sf_status sf_world_create(const sf_world_desc *desc, const sf_params *params, sf
     sf::DBuf<float> d_pose;
     SF_CUDA(upload(d_pose, pose, st));
     SF_CUDA(w->b_pos.alloc(nb)); SF_CUDA(w->b_q.alloc(nb)); SF_CUDA(w->b_v.alloc(nb)); SF_CUDA(w->b_w.alloc(nb));
-    SF_CUDA(w->b_vpre.alloc(nb)); SF_CUDA(w->b_wpre.alloc(nb));
     SF_CUDA(w->b_rot.alloc((size_t)nb * 9)); SF_CUDA(w->b_iil.alloc((size_t)nb * 9)); SF_CUDA(w->b_iiw.alloc((size_t)nb * 9));
     SF_CUDA(w->b_m.alloc(nb)); SF_CUDA(w->b_im.alloc(nb)); SF_CUDA(w->b_rad.alloc(nb)); SF_CUDA(w->b_sleep.alloc(nb));
     SF_CUDA(w->b_maxr.alloc(nb));
@@ -978,7 +977,6 @@ sf_status sf_pool_create(uint32_t n_slots, const sf_pool_slot *slots, const sf_p
     std::vector<uint32_t> k_body(nd, w->sentinel);
     SF_CUDA(upload(w->k_body, k_body, st));
     SF_CUDA(w->b_pos.alloc(nb)); SF_CUDA(w->b_q.alloc(nb)); SF_CUDA(w->b_v.alloc(nb)); SF_CUDA(w->b_w.alloc(nb));
-    SF_CUDA(w->b_vpre.alloc(nb)); SF_CUDA(w->b_wpre.alloc(nb));
     SF_CUDA(w->b_rot.alloc((size_t)nb * 9)); SF_CUDA(w->b_iil.alloc((size_t)nb * 9)); SF_CUDA(w->b_iiw.alloc((size_t)nb * 9));
     SF_CUDA(w->b_m.alloc(nb)); SF_CUDA(w->b_im.alloc(nb)); SF_CUDA(w->b_rad.alloc(nb)); SF_CUDA(w->b_sleep.alloc(nb));
     SF_CUDA(w->b_maxr.alloc(nb));
