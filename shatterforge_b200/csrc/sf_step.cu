@@ -39,6 +39,7 @@ struct StepState {
     uint32_t n_awk = 0;
     bool use_sparse = false, last_sparse = false;
     DBuf<uint32_t> bstart;          // the hash table: per (active scene, bucket) count, then start (+1 for the end)
+    DBuf<uint32_t> bsig;            // per (active scene, bucket) a 16-bit signature
     DBuf<float4> srec;
     DBuf<uint2> sent;
     DBuf<uint4> slot_id;
@@ -139,7 +140,7 @@ static void prof_mark(sf_world *w) {
 }
 
 enum { DV_CONTACTS = 0, DV_MANIFOLDS = 1, DV_COLORS = 2, DV_ROUNDS = 3, DV_WL0 = 4, DV_WL1 = 5, DV_WL2 = 6,
-       DV_ALIVE = 7, DV_AWAKE = 8, DV_ISLANDS = 9, DV_PAIRS = 10, DV_AWK = 11, DV_INC = 12, DV_NBIG = 13, DV_KEPT = 14, DV_MAXDEG = 15, DV_N = 16 };
+       DV_ALIVE = 7, DV_AWAKE = 8, DV_ISLANDS = 9, DV_PAIRS = 10, DV_AWK = 11, DV_INC = 12, DV_NBIG = 13, DV_KEPT = 14, DV_MAXDEG = 15, DV_RUN = 16, DV_N = 17 };
 constexpr int JDS_K = 32;   // the largest manifold chunk: the depth of the solve's contact layout
 
 // ---------------------------------------------------------------- pose cache
@@ -185,6 +186,23 @@ __global__ void k_brick_pos(uint32_t nd, const uint32_t *list, const uint32_t *k
 }
 
 __device__ __forceinline__ int floor_cell(float x) { return __float2int_rz(floorf(x / S)); }
+
+// The signature bit of a cell: one of 16, by the region of 16^3 cells it lies in. A brick's walk asks a bucket for the
+// bits of the regions within two cells of it (a brick that touches it lies in one of them), so a bucket filled by other
+// parts of the scene alone is mostly passed over without a read.
+constexpr int SIG_SHIFT = 4;
+__device__ __forceinline__ uint32_t region_sig(int rx, int ry, int rz) {
+    const uint32_t h = (uint32_t)rx * 0x9E3779B1u ^ (uint32_t)ry * 0x85EBCA6Bu ^ (uint32_t)rz * 0xC2B2AE35u;
+    return 1u << ((h ^ (h >> 13) ^ (h >> 22)) & 15u);
+}
+__device__ __forceinline__ uint32_t cell_sig(int x, int y, int z) { return region_sig(x >> SIG_SHIFT, y >> SIG_SHIFT, z >> SIG_SHIFT); }
+__device__ __forceinline__ uint32_t near_sig(int x, int y, int z) {
+    uint32_t m = 0;
+    for (int rz = (z - 2) >> SIG_SHIFT; rz <= (z + 2) >> SIG_SHIFT; rz++)
+        for (int ry = (y - 2) >> SIG_SHIFT; ry <= (y + 2) >> SIG_SHIFT; ry++)
+            for (int rx = (x - 2) >> SIG_SHIFT; rx <= (x + 2) >> SIG_SHIFT; rx++) m |= region_sig(rx, ry, rz);
+    return m;
+}
 
 // The hash holds the bricks a bucket walk can meet: every awake brick, and each other live brick whose bucket is one
 // of the 27 around an awake brick (gen_contacts walks only those buckets, so a brick outside them is never read; the
@@ -237,13 +255,14 @@ __global__ void k_mark_buckets(const uint32_t *n_p, const uint32_t *awk, const u
 // the counts gives every bucket's start (the table is then CSR: bucket k holds [start[k], start[k + 1])), the bricks
 // are placed by start + rank (k_hash_place), and each bucket's few entries are put in ascending brick-id order
 // (k_hash_order), which is the order a walk from the highest id down needs (the reference's chain order).
+// Beside the counts, a 16-bit signature a bucket (two to a word): the bits of the regions its bricks lie in (cell_sig).
 // A brick goes in when it is alive; in the sparse form (most bricks asleep) only when it is awake, its scene has more
 // than 1/8 of its bricks awake, or its bucket is one a walk can reach (gen_contacts walks only the 27 buckets around
 // an awake brick, so leaving other bricks out changes no walk).
 __global__ void k_hash_count(uint32_t nd, const uint32_t *list, const uint32_t *kbody, const uint32_t *bscene,
                              const uint32_t *scene_act, const uint32_t *scene_awake, const uint32_t *scene_bricks,
                              const uint8_t *alive, const uint8_t *asleep, const float4 *wpos, const uint32_t *bits,
-                             uint32_t *cnt, uint32_t *tkey, uint32_t *trank) {
+                             uint32_t *cnt, uint32_t *sig, uint32_t *tkey, uint32_t *trank) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nd) return;
     const uint32_t i = pick(list, t);
@@ -252,12 +271,14 @@ __global__ void k_hash_count(uint32_t nd, const uint32_t *list, const uint32_t *
     if (alive[b]) {
         const float4 p = wpos[i];
         const uint32_t sk = scene_act[bscene[b]];
-        const uint32_t h = hkey(floor_cell(p.x), floor_cell(p.y), floor_cell(p.z));
+        const int hx = floor_cell(p.x), hy = floor_cell(p.y), hz = floor_cell(p.z);
+        const uint32_t h = hkey(hx, hy, hz);
         const bool in = !bits || !asleep[b] || scene_full(scene_awake, scene_bricks, sk) ||
                         ((bits[(size_t)sk * (HSIZE / 32) + (h >> 5)] >> (h & 31)) & 1u);
         if (in) {
             key = sk * HSIZE + h;
             rank = atomicAdd(&cnt[key], 1u);
+            if (sig) atomicOr(&sig[key >> 1], cell_sig(hx, hy, hz) << (16 * (key & 1)));
         }
     }
     tkey[t] = key;
@@ -289,14 +310,12 @@ __device__ __forceinline__ uint32_t pack_wcell(int x, int y, int z) {
     x = min(max(x + 1024, 0), 2047); y = min(max(y + 512, 0), 1023); z = min(max(z + 1024, 0), 2047);
     return (uint32_t)x | ((uint32_t)y << 11) | ((uint32_t)z << 21);
 }
-// true when the packed cells differ by at most 2 in every coordinate: two brick centres closer than 2 RB = 0.54 m
-// (1.08 cells) always are, so a bucket entry that fails this cannot touch the brick and is skipped unread
-__device__ __forceinline__ bool wcell_near(uint32_t a, uint32_t b) {
-    const int dx = (int)(a & 2047u) - (int)(b & 2047u);
-    const int dy = (int)((a >> 11) & 1023u) - (int)((b >> 11) & 1023u);
-    const int dz = (int)(a >> 21) - (int)(b >> 21);
-    return (uint32_t)(dx + 2) <= 4u && (uint32_t)(dy + 2) <= 4u && (uint32_t)(dz + 2) <= 4u;
-}
+// Two brick centres closer than 2 RB = 0.54 m (1.08 cells) lie in cells that differ by at most 2 in every coordinate. The
+// packed difference plus 3 in every field then has fields of 1 to 5 and no carry between them, so an entry whose sum has
+// any bit above the fields' lowest three cannot touch the brick and is skipped unread (one that passes may still be far).
+constexpr uint32_t WCELL_3 = 3u | (3u << 11) | (3u << 21), WCELL_FAR = ~(7u | (7u << 11) | (7u << 21));
+__device__ __forceinline__ uint32_t wcell_base(uint32_t mine) { return WCELL_3 - mine; }
+__device__ __forceinline__ bool wcell_near(uint32_t base, uint32_t other) { return ((base + other) & WCELL_FAR) == 0; }
 
 // Packed bucket entries in sorted order: world position and brick id (srec), and the packed world cell with the body
 // id, its asleep bit (31) and the removed-brick bit (30) (sent), so a bucket walk reads contiguous arrays: the 8-byte
@@ -324,6 +343,7 @@ struct ContactArgs {
     const float4 *wpos, *v, *w;
     const float *rot, *rad;
     const uint32_t *bstart;            // per (active scene, bucket): first entry; the next bucket's start ends it
+    const uint32_t *sig;               // per (active scene, bucket): 16-bit signature
     const float4 *srec;
     const uint2 *sent;
     uint32_t *ccount;
@@ -340,12 +360,21 @@ struct ContactArgs {
 constexpr int CSLOTS = 12;
 constexpr int WALK = 8;        // bucket entries whose packed words one brick loads together
 
-// gen_contacts for one brick of an awake body (src/lib.rs:1410-1468), contacts emitted in the reference's order.
+// A scene's bucket table in shared memory: starts relative to the start of their group of 64 buckets, and signatures.
+struct BucketTab {
+    uint16_t start[HSIZE];
+    uint16_t sig[HSIZE];
+    uint32_t base[HSIZE / 64 + 1];
+    uint32_t wide;                     // a group holds more entries than 16 bits count: starts are read from memory
+    __device__ __forceinline__ uint32_t first(uint32_t h) const { return base[h >> 6] + start[h]; }
+    __device__ __forceinline__ uint32_t end(uint32_t h) const { return (h & 63u) == 63u ? base[(h >> 6) + 1] : first(h + 1); }
+};
+
+// gen_contacts for one brick of an awake body (src/lib.rs:1410-1468), contacts emitted in the reference's order: ground
+// and static cells (gen_fixed), then hashed neighbours (gen_hash, or the table form below).
 template <bool WAKE, class Emit>
-__device__ __forceinline__ void gen_brick(const ContactArgs &A, uint32_t i, uint32_t a, Emit &&emit) {
+__device__ __forceinline__ void gen_fixed(const ContactArgs &A, uint32_t i, uint32_t a, V3 p, Emit &&emit) {
     const uint32_t sc = A.bscene[a];
-    const float4 p4 = A.wpos[i];
-    const V3 p = v3(p4.x, p4.y, p4.z);
     // ground: the brick's 8 cube corners below y = 0 (src/lib.rs:1415-1421)
     if (p.y < 0.5f) {
         float r[9];
@@ -408,76 +437,146 @@ __device__ __forceinline__ void gen_brick(const ContactArgs &A, uint32_t i, uint
                     }
         }
     }
-    // hashed neighbours in the 27 buckets around the brick (src/lib.rs:1441-1466); a bucket walked from its highest
-    // brick id down is the reference's chain order
-    {
-        const int hx = floor_cell(p.x), hy = floor_cell(p.y), hz = floor_cell(p.z);
-        const uint32_t sk = A.scene_act[sc];
-        float speed = 0.0f;
+}
+
+// one bucket entry near enough to touch (its packed word's second half, its place) against brick i of body a at p
+template <bool WAKE, class Emit>
+__device__ __forceinline__ void gen_meet(const ContactArgs &A, uint32_t i, uint32_t a, V3 p, uint32_t info, uint32_t at, Emit &&emit) {
+    const uint32_t bj = info & 0x3FFFFFFFu;
+    if (bj == a || (info & 0x40000000u)) return;
+    const float4 rec = A.srec[at];
+    const uint32_t j = __float_as_uint(rec.w);
+    const bool other_awake = !(info & 0x80000000u);
+    if (other_awake && j < i) return;
+    const V3 pj = v3(rec.x, rec.y, rec.z);
+    const V3 d = sub(p, pj);
+    const float dd = dot(d, d);
+    if (dd >= 4.0f * RB * RB || dd < 1e-10f) return;
+    const float dist = sqrt_rn(dd);
+    const V3 nn = mul(d, div_rn(1.0f, dist));
+    const V3 cp = madd(pj, nn, dist * 0.5f);
+    if (WAKE && A.sup) {
+        if (nn.y > 0.3f) A.sup[i] = A.frame;
+        else if (nn.y < -0.3f) A.sup[j] = A.frame;
+    }
+    if (other_awake) emit(bj, bj, j, cp, nn, 2.0f * RB - dist);
+    else {
         if (WAKE) {
             const float4 vv = A.v[a], ww = A.w[a];
-            speed = len(v3(vv.x, vv.y, vv.z)) + len(v3(ww.x, ww.y, ww.z)) * A.rad[a] * 0.5f;
+            if (len(v3(vv.x, vv.y, vv.z)) + len(v3(ww.x, ww.y, ww.z)) * A.rad[a] * 0.5f > 0.7f) A.wake[bj] = 1;
         }
-        const float lim2 = 4.0f * RB * RB;
-        const uint32_t mycell = pack_wcell(hx, hy, hz);
-        const uint32_t *bst = A.bstart + (size_t)sk * HSIZE;
-        for (int dz = -1; dz <= 1; dz++) {
-            // The layer's nine buckets are walked as one sequence: bucket c (the reference's dy, dx order) from its
-            // highest brick id down; entry t of the sequence lies in bucket c with pre[c] <= t < pre[c + 1]. The
-            // nine buckets' bounds are fetched together, then the packed (cell, body) words of WALK entries at a time, so a
-            // brick waits on a few rounds of loads per layer instead of one per entry; only entries near enough to
-            // touch (a full bucket holds mostly other cells that share its hash) go on to the position record.
-            uint32_t hi[9], pre[10];
-            pre[0] = 0;
+        emit(STATIC, bj, j, cp, nn, 2.0f * RB - dist);
+    }
+}
+
+// hashed neighbours in the 27 buckets around the brick (src/lib.rs:1441-1466); a bucket walked from its highest brick id
+// down is the reference's chain order
+template <bool WAKE, class Emit>
+__device__ __forceinline__ void gen_hash(const ContactArgs &A, uint32_t i, uint32_t a, V3 p, Emit &&emit) {
+    const int hx = floor_cell(p.x), hy = floor_cell(p.y), hz = floor_cell(p.z);
+    const uint32_t mycell = wcell_base(pack_wcell(hx, hy, hz));
+    const uint32_t *bst = A.bstart + (size_t)A.scene_act[A.bscene[a]] * HSIZE;
+    for (int dz = -1; dz <= 1; dz++) {
+        // The layer's nine buckets are walked as one sequence: bucket c (the reference's dy, dx order) from its
+        // highest brick id down; entry t of the sequence lies in bucket c with pre[c] <= t < pre[c + 1]. The
+        // nine buckets' bounds are fetched together, then the packed (cell, body) words of WALK entries at a time, so a
+        // brick waits on a few rounds of loads per layer instead of one per entry; only entries near enough to
+        // touch (a full bucket holds mostly other cells that share its hash) go on to the position record.
+        uint32_t hi[9], pre[10];
+        pre[0] = 0;
 #pragma unroll
-            for (int c = 0; c < 9; c++) {
-                const uint32_t h = hkey(hx + (c % 3) - 1, hy + (c / 3) - 1, hz + dz);
-                const uint32_t lo = bst[h];
-                hi[c] = bst[h + 1];
-                pre[c + 1] = pre[c] + (hi[c] - lo);
+        for (int c = 0; c < 9; c++) {
+            const uint32_t h = hkey(hx + (c % 3) - 1, hy + (c / 3) - 1, hz + dz);
+            const uint32_t lo = bst[h];
+            hi[c] = bst[h + 1];
+            pre[c + 1] = pre[c] + (hi[c] - lo);
+        }
+        const uint32_t n = pre[9];
+        for (uint32_t b0 = 0; b0 < n; b0 += WALK) {
+            uint2 e[WALK];
+            uint32_t qq[WALK];
+#pragma unroll
+            for (int u = 0; u < WALK; u++) {
+                const uint32_t t = b0 + u;
+                uint32_t h = hi[0], p0 = pre[0];
+#pragma unroll
+                for (int k = 1; k < 9; k++) if (t >= pre[k]) { h = hi[k]; p0 = pre[k]; }
+                qq[u] = h - 1u - (t - p0);
+                e[u] = t < n ? A.sent[qq[u]] : make_uint2(0u, 0u);
             }
-            const uint32_t n = pre[9];
-            for (uint32_t b0 = 0; b0 < n; b0 += WALK) {
-                uint2 e[WALK];
-                uint32_t qq[WALK];
 #pragma unroll
-                for (int u = 0; u < WALK; u++) {
-                    const uint32_t t = b0 + u;
-                    uint32_t h = hi[0], p0 = pre[0];
-#pragma unroll
-                    for (int k = 1; k < 9; k++) if (t >= pre[k]) { h = hi[k]; p0 = pre[k]; }
-                    qq[u] = h - 1u - (t - p0);
-                    e[u] = t < n ? A.sent[qq[u]] : make_uint2(0u, 0u);
-                }
-#pragma unroll
-                for (int u = 0; u < WALK; u++) {
-                    if (b0 + u >= n) break;
-                    if (!wcell_near(mycell, e[u].x)) continue;
-                    const uint32_t info = e[u].y;
-                    const uint32_t bj = info & 0x3FFFFFFFu;
-                    if (bj == a || (info & 0x40000000u)) continue;
-                    const float4 rec = A.srec[qq[u]];
-                    const uint32_t j = __float_as_uint(rec.w);
-                    const bool other_awake = !(info & 0x80000000u);
-                    if (other_awake && j < i) continue;
-                    const V3 pj = v3(rec.x, rec.y, rec.z);
-                    const V3 d = sub(p, pj);
-                    const float dd = dot(d, d);
-                    if (dd >= lim2 || dd < 1e-10f) continue;
-                    const float dist = sqrt_rn(dd);
-                    const V3 nn = mul(d, div_rn(1.0f, dist));
-                    const V3 cp = madd(pj, nn, dist * 0.5f);
-                    if (WAKE && A.sup) {
-                        if (nn.y > 0.3f) A.sup[i] = A.frame;
-                        else if (nn.y < -0.3f) A.sup[j] = A.frame;
-                    }
-                    if (other_awake) emit(bj, bj, j, cp, nn, 2.0f * RB - dist);
-                    else {
-                        if (WAKE && speed > 0.7f) A.wake[bj] = 1;
-                        emit(STATIC, bj, j, cp, nn, 2.0f * RB - dist);
-                    }
-                }
+            for (int u = 0; u < WALK; u++) {
+                if (b0 + u >= n) break;
+                if (!wcell_near(mycell, e[u].x)) continue;
+                gen_meet<WAKE>(A, i, a, p, e[u].y, qq[u], emit);
             }
+        }
+    }
+}
+
+// The same from the scene's table, for a warp's 32 bricks together (on: the lane has one). A lane finds the buckets whose
+// signature has one of the regions around its brick; then the warp's lanes share all those buckets out and look for an
+// entry of another body within two cells of the brick whose bucket it is, and each lane walks only its buckets that have
+// one. queue: 27 x 32 entries and 32 words of the warp's own.
+struct WarpQueue { uint32_t found[32]; uint16_t item[27 * 32]; };
+template <class Emit>
+__device__ __forceinline__ void gen_hash_tab(const ContactArgs &A, bool on, uint32_t i, uint32_t a, V3 p, uint32_t sk,
+                                             const BucketTab *tab, WarpQueue *queue, Emit &&emit) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const int hx = floor_cell(p.x), hy = floor_cell(p.y), hz = floor_cell(p.z);
+    const uint32_t mycell = wcell_base(pack_wcell(hx, hy, hz));
+    const uint32_t *bst = A.bstart + (size_t)sk * HSIZE;
+    const bool wide = tab->wide != 0;
+    auto key_of = [](int x, int y, int z, uint32_t c) {   // the bucket of the c-th of the 27 cells around
+        const uint32_t dz = (c * 57u) >> 9, r = c - 9u * dz, dy = (r * 11u) >> 5, dx = r - 3u * dy;
+        return hkey(x - 1 + (int)dx, y - 1 + (int)dy, z - 1 + (int)dz);
+    };
+    // hkey, whose terms of one axis do not depend on the others
+    auto kx = [](int x) { return (uint32_t)x * 73856093u; };
+    auto ky = [](int y) { return (uint32_t)y * 19349663u; };
+    auto kz = [](int z) { return (uint32_t)z * 83492791u; };
+    uint32_t pass = 0;
+    if (on) {
+        const uint32_t want = near_sig(hx, hy, hz);
+        const uint32_t X[3] = {kx(hx - 1), kx(hx), kx(hx + 1)}, Y[3] = {ky(hy - 1), ky(hy), ky(hy + 1)};
+        const uint32_t Z[3] = {kz(hz - 1), kz(hz), kz(hz + 1)};
+#pragma unroll
+        for (int c = 0; c < 27; c++)
+            if (tab->sig[(X[c % 3] ^ Y[(c / 3) % 3] ^ Z[c / 9]) & (HSIZE - 1)] & want) pass |= 1u << c;
+    }
+    const uint32_t mine = __popc(pass);
+    uint32_t before = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, before, o); if (lane >= (uint32_t)o) before += y; }
+    const uint32_t total = __shfl_sync(0xffffffffu, before, 31);
+    before -= mine;
+    __syncwarp();
+    for (uint32_t rest = pass; rest; rest &= rest - 1) queue->item[before++] = (uint16_t)((__ffs(rest) - 1) << 5 | lane);
+    queue->found[lane] = 0;
+    __syncwarp();
+    for (uint32_t r = 0; r < total; r += 32) {
+        const bool has = r + lane < total;
+        const uint32_t it = has ? queue->item[r + lane] : 0u, of = it & 31u, c = it >> 5;
+        const int ox = __shfl_sync(0xffffffffu, hx, of), oy = __shfl_sync(0xffffffffu, hy, of), oz = __shfl_sync(0xffffffffu, hz, of);
+        const uint32_t cell = __shfl_sync(0xffffffffu, mycell, of), body = __shfl_sync(0xffffffffu, a, of);
+        if (!has) continue;
+        const uint32_t h = key_of(ox, oy, oz, c);
+        uint32_t q = wide ? bst[h] : tab->first(h);
+        const uint32_t q1 = wide ? bst[h + 1] : tab->end(h);
+        bool hit = false;
+        for (; q < q1; q++) {
+            const uint2 e = A.sent[q];
+            hit |= wcell_near(cell, e.x) && (e.y & 0x3FFFFFFFu) != body;
+        }
+        if (hit) atomicOr(&queue->found[of], 1u << c);
+    }
+    __syncwarp();
+    for (uint32_t rest = queue->found[lane]; rest; rest &= rest - 1) {
+        const uint32_t h = key_of(hx, hy, hz, __ffs(rest) - 1);
+        const uint32_t lo = wide ? bst[h] : tab->first(h);
+        for (uint32_t q = wide ? bst[h + 1] : tab->end(h); q-- > lo;) {
+            const uint2 e = A.sent[q];
+            if (wcell_near(mycell, e.x)) gen_meet<true>(A, i, a, p, e.y, q, emit);
         }
     }
 }
@@ -486,25 +585,112 @@ __device__ __forceinline__ void gen_brick(const ContactArgs &A, uint32_t i, uint
 #ifndef SF_GEN_BLOCKS_PER_SM
 #define SF_GEN_BLOCKS_PER_SM 6   // 80 registers (a few spilled): measured faster than 4 or 5 blocks an SM
 #endif
+// the place of a brick's n-th contact in the slots
+struct SlotEmit {
+    const ContactArgs &A;
+    uint32_t t, n;
+    __device__ __forceinline__ void operator()(uint32_t b, uint32_t bo, uint32_t bb, V3 cp, V3 nn, float depth) {
+        if (n < CSLOTS) {
+            const size_t o = (size_t)n * A.nd + t;
+            A.slot_id[o] = make_uint4(b, bo, bb, 0u);
+            A.slot_p[o] = make_float4(cp.x, cp.y, cp.z, depth);
+            A.slot_n[o] = make_float4(nn.x, nn.y, nn.z, 0.0f);
+        }
+        n++;
+    }
+};
 __global__ void __launch_bounds__(128, SF_GEN_BLOCKS_PER_SM) k_contacts_gen(ContactArgs A) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= A.nd) return;
     const uint32_t i = pick(A.list, t);
     const uint32_t a = A.kbody[i];
     if (!A.alive[a] || A.asleep[a]) { A.ccount[t] = 0; return; }
-    uint32_t n = 0;
-    const size_t nd = A.nd;
-    auto emit = [&](uint32_t b, uint32_t bo, uint32_t bb, V3 cp, V3 nn, float depth) {
-        if (n < CSLOTS) {
-            const size_t o = (size_t)n * nd + t;
-            A.slot_id[o] = make_uint4(b, bo, bb, 0u);
-            A.slot_p[o] = make_float4(cp.x, cp.y, cp.z, depth);
-            A.slot_n[o] = make_float4(nn.x, nn.y, nn.z, 0.0f);
+    SlotEmit emit{A, t, 0};
+    const float4 p4 = A.wpos[i];
+    const V3 p = v3(p4.x, p4.y, p4.z);
+    gen_fixed<true>(A, i, a, p, emit);
+    gen_hash<true>(A, i, a, p, emit);
+    A.ccount[t] = emit.n;
+}
+// The same with the scene's bucket table in shared memory: read from memory, the 27 buckets' bounds and their entries,
+// mostly bricks of elsewhere that share the hash, were some 50 L2 sectors a brick, which is what bounded the pass. A block
+// takes runs of GEN_TAB_RUN consecutive bricks and loads the table of each scene they lie in (bricks are listed scene by
+// scene), and a warp 32 of them at a time. What bounds it now is instruction issue (some 2,000 a warp, half the lanes on).
+// Per launch on the 256-scene mix (4.38M bricks) in free fall 989 -> 505 us, at the contact peak 1,642 -> 1,000 us; a world
+// of 12,000 bricks takes 35 us against the other form's 26, 97,000 bricks in one scene 56 against 62.
+constexpr int GEN_TAB_T = 1024;
+constexpr size_t GEN_TAB_SMEM = sizeof(BucketTab) + (GEN_TAB_T / 32) * sizeof(WarpQueue);
+constexpr uint32_t GEN_TAB_RUNS = 4;   // runs a block, about
+constexpr uint32_t GEN_TAB_MIN = 256, GEN_TAB_ALL = 65536;   // bricks a scene on average, and in all, from which it is taken
+__global__ void __launch_bounds__(GEN_TAB_T) k_contacts_gen_tab(ContactArgs A, uint32_t run, uint32_t K, const uint4 *seg,
+                                                                const uint32_t *awk_pos, uint32_t nd_act, uint32_t *runs) {
+    extern __shared__ __align__(16) unsigned char s_tab[];
+    __shared__ uint32_t s_next, s_run;               // the segment's bricks handed out so far; this block's run
+    BucketTab *tab = reinterpret_cast<BucketTab *>(s_tab);
+    WarpQueue *queue = reinterpret_cast<WarpQueue *>(s_tab + sizeof(BucketTab)) + threadIdx.x / 32;
+    const uint32_t lane = threadIdx.x & 31u;
+    // where the k-th active scene's bricks begin in the list (the awake ones' list has its own places)
+    auto begins = [&](uint32_t k) -> uint32_t { return k >= K || seg[k].w >= nd_act ? A.nd : awk_pos ? awk_pos[seg[k].w] : seg[k].w; };
+    uint32_t loaded = NONE;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_run = atomicAdd(runs, 1u);
+        __syncthreads();
+        const uint64_t r0 = (uint64_t)s_run * run;
+        if (r0 >= A.nd) break;
+        const uint32_t r1 = (uint32_t)min((uint64_t)A.nd, r0 + run);
+        uint32_t k = 0, hi = K;                      // the last scene that begins at or before r0
+        while (hi - k > 1) {
+            const uint32_t mid = (k + hi) >> 1;
+            if (begins(mid) <= r0) k = mid; else hi = mid;
         }
-        n++;
-    };
-    gen_brick<true>(A, i, a, emit);
-    A.ccount[t] = n;
+        for (uint32_t t0 = (uint32_t)r0; t0 < r1; k++) {
+            const uint32_t t1 = min(r1, begins(k + 1));
+            if (t1 <= t0) continue;                  // (a scene without bricks in the list)
+            __syncthreads();
+            if (threadIdx.x == 0) { s_next = t0; tab->wide = loaded == k ? tab->wide : 0u; }
+            __syncthreads();
+            if (loaded != k) {
+                const uint32_t *bst = A.bstart + (size_t)k * HSIZE;
+                const uint32_t *bsig = A.sig + (size_t)k * (HSIZE / 2);
+                for (uint32_t q = threadIdx.x; q < HSIZE / 2; q += GEN_TAB_T) reinterpret_cast<uint32_t *>(tab->sig)[q] = bsig[q];
+                for (uint32_t q = threadIdx.x; q < HSIZE; q += GEN_TAB_T) {
+                    const uint32_t d = bst[q] - bst[q & ~63u];
+                    tab->start[q] = (uint16_t)d;
+                    if (d > 0xFFFFu) tab->wide = 1;
+                }
+                for (uint32_t q = threadIdx.x; q <= HSIZE / 64; q += GEN_TAB_T) tab->base[q] = bst[q * 64];
+                loaded = k;
+                __syncthreads();
+            }
+            for (;;) {                               // 32 bricks a warp at a time, until the segment's are handed out
+                uint32_t t = 0;
+                if (lane == 0) t = atomicAdd(&s_next, 32u);
+                t = __shfl_sync(0xffffffffu, t, 0);
+                if (t >= t1) break;
+                t += lane;
+                uint32_t i = 0, a = 0;
+                bool on = false;
+                if (t < t1) {
+                    i = pick(A.list, t);
+                    a = A.kbody[i];
+                    on = A.alive[a] && !A.asleep[a];
+                    if (!on) A.ccount[t] = 0;
+                }
+                SlotEmit emit{A, t, 0};
+                V3 p = v3(0.0f, 0.0f, 0.0f);
+                if (on) {
+                    const float4 p4 = A.wpos[i];
+                    p = v3(p4.x, p4.y, p4.z);
+                    gen_fixed<true>(A, i, a, p, emit);
+                }
+                __syncwarp();
+                if (__any_sync(0xffffffffu, on)) gen_hash_tab(A, on, i, a, p, k, tab, queue, emit);
+                if (on) A.ccount[t] = emit.n;
+            }
+            t0 = t1;
+        }
+    }
 }
 
 // pass 2: each brick's contacts to their place in the list; a brick with more than CSLOTS regenerates them
@@ -537,7 +723,10 @@ __global__ void __launch_bounds__(128) k_contacts_place(ContactArgs A) {
         A.L_n[t] = make_float4(nn.x, nn.y, nn.z, depth);
         k++;
     };
-    gen_brick<false>(A, i, a, emit);
+    const float4 p4 = A.wpos[i];
+    const V3 p = v3(p4.x, p4.y, p4.z);
+    gen_fixed<false>(A, i, a, p, emit);
+    gen_hash<false>(A, i, a, p, emit);
 }
 
 __global__ void k_body_nc(uint32_t nc, const uint32_t *L_a, const uint32_t *L_b, uint32_t *bnc) {
@@ -1852,7 +2041,8 @@ sf_status step_create(sf_world *w) {
     SF_CUDA(S->aw_flag.alloc(nd)); SF_CUDA(S->awk_pos.alloc(nd)); SF_CUDA(S->awk_list.alloc(nd));
     SF_CUDA(S->bucket_bits.alloc((size_t)nsc * (HSIZE / 32)));
     SF_CUDA(S->scene_awake.alloc(nsc)); SF_CUDA(S->scene_bricks.alloc(nsc));
-    SF_CUDA(S->bstart.alloc((size_t)nsc * HSIZE + 1));
+    SF_CUDA(S->bstart.alloc((size_t)nsc * HSIZE + 1)); SF_CUDA(S->bsig.alloc((size_t)nsc * (HSIZE / 2)));
+    SF_CUDA(cudaFuncSetAttribute(k_contacts_gen_tab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEN_TAB_SMEM));
     SF_CUDA(S->srec.alloc(nd)); SF_CUDA(S->sent.alloc(nd));
     SF_CUDA(S->slot_id.alloc((size_t)nd * CSLOTS)); SF_CUDA(S->slot_p.alloc((size_t)nd * CSLOTS)); SF_CUDA(S->slot_n.alloc((size_t)nd * CSLOTS));
     SF_CUDA(S->ccount.alloc((size_t)nd + 1)); SF_CUDA(S->coff.alloc((size_t)nd + 1));
@@ -2090,10 +2280,13 @@ static sf_status substep(sf_world *w, float h) {
     }
     // the hash table (counting sort into the buckets; see k_hash_count)
     SF_CUDA(cudaMemsetAsync(S->bstart.p, 0, nbk * 4, s));
+    // (a scene's table is loaded whole, 192 KB: see k_contacts_gen_tab for both forms' times)
+    const bool tab = nd >= GEN_TAB_ALL && (uint64_t)nd >= (uint64_t)S->act.size() * GEN_TAB_MIN;
+    if (tab) SF_CUDA(cudaMemsetAsync(S->bsig.p, 0, nbk * 2, s));
     k_hash_count<<<grid_for(nd, 256), 256, 0, s>>>(nd, klist, w->k_body.p, w->b_scene.p, S->scene_act.p,
                                                    sparse ? S->scene_awake.p : nullptr, S->scene_bricks.p, w->b_alive.p,
                                                    w->b_asleep.p, w->k_wpos.p, sparse ? S->bucket_bits.p : nullptr,
-                                                   S->bstart.p, S->ckey.p, S->ckey_alt.p);
+                                                   S->bstart.p, tab ? S->bsig.p : nullptr, S->ckey.p, S->ckey_alt.p);
     SF_CUDA(exclusive_scan_u32(S->bstart.p, S->bstart.p, nbk, S->bstart.p + nbk, S->wk, s));
     k_hash_place<<<grid_for(nd, 256), 256, 0, s>>>(nd, klist, S->ckey.p, S->ckey_alt.p, S->bstart.p, S->cval.p);
     k_hash_order<<<grid_for(nbk, 256), 256, 0, s>>>((uint32_t)nbk, S->bstart.p, S->cval.p);
@@ -2112,7 +2305,7 @@ static sf_status substep(sf_world *w, float h) {
     C.nd = n_awk; C.list = clist; C.scene_act = S->scene_act.p;
     C.sbox = w->sbox.p; C.kbody = w->k_body.p; C.bscene = w->b_scene.p; C.ctab = w->ctab.p; C.cpool = w->cpool.p;
     C.alive = w->b_alive.p; C.asleep = w->b_asleep.p; C.smat = w->s_mat.p; C.wpos = w->k_wpos.p;
-    C.v = w->b_v.p; C.w = w->b_w.p; C.rot = w->b_rot.p; C.rad = w->b_rad.p; C.bstart = S->bstart.p; C.srec = S->srec.p;
+    C.v = w->b_v.p; C.w = w->b_w.p; C.rot = w->b_rot.p; C.rad = w->b_rad.p; C.bstart = S->bstart.p; C.sig = S->bsig.p; C.srec = S->srec.p;
     C.sent = S->sent.p; C.ccount = S->ccount.p; C.coff = S->coff.p; C.wake = w->b_wake.p;
     C.sup = w->k_sup.p; C.frame = w->frame;
     C.slot_id = S->slot_id.p; C.slot_p = S->slot_p.p; C.slot_n = S->slot_n.p;
@@ -2131,7 +2324,13 @@ static sf_status substep(sf_world *w, float h) {
         }
     }
     if (g0) cudaEventRecord(g0, s);
-    if (n_awk) k_contacts_gen<<<grid_for(n_awk, 128), 128, 0, s>>>(C);
+    if (tab && n_awk >= GEN_TAB_ALL) {
+        // runs taken in turn, about GEN_TAB_RUNS a block (an even load without many table loads)
+        const uint32_t run = std::max<uint32_t>(GEN_TAB_T, (n_awk / (GEN_TAB_RUNS * w->sms) + 31) / 32 * 32);
+        SF_CUDA(cudaMemsetAsync(S->dev.p + DV_RUN, 0, 4, s));
+        k_contacts_gen_tab<<<std::min<unsigned>(w->sms, grid_for(n_awk, run)), GEN_TAB_T, GEN_TAB_SMEM, s>>>(
+            C, run, (uint32_t)S->act.size(), S->seg.p, sparse ? S->awk_pos.p : nullptr, nd, S->dev.p + DV_RUN);
+    } else if (n_awk) k_contacts_gen<<<grid_for(n_awk, 128), 128, 0, s>>>(C);
     if (g1) cudaEventRecord(g1, s);
     SF_CUDA(exclusive_scan_u32(S->ccount.p, S->coff.p, n_awk, S->dev.p + DV_CONTACTS, S->wk, s));
     SF_CUDA(cudaMemcpyAsync(S->h_dev, S->dev.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
