@@ -1329,6 +1329,423 @@ __global__ void k_col_verify(const uint32_t *nm_p, const uint32_t *man_a, const 
     if (b != STATIC && (atomicOr(&vmasks[(size_t)b * mw + (c >> 5)], bit) & bit)) atomicOr(err, (unsigned)ERR_VERIFY_COLOR);
 }
 
+// ---------------------------------------------------------------- small substeps: manifolds and colours in one block
+// The manifolds of a substep of at most SMALL_MAX contacts, their colours and the contact layout, by one block: the
+// contacts sorted by pair, reduced, cut into chunks, coloured and listed as the kernels above do it (the same manifolds,
+// colours and rounds; only the order inside a list's bucket is free). Those are some forty-five launches, which is what
+// bounds them on few contacts; the one block is bound by the latency of its phases (2 to 4 us each, a colouring round 2).
+// Against those launches: 1,300 contacts (12 rounds) 276 -> 59 us, 2,980 (13) 332 -> 82, 3,450 with reduction 264 -> 58,
+// 7,580 (4) 230 -> 56 us.
+constexpr int SMALL_T = 1024, SMALL_ITEMS = 8;
+constexpr uint32_t SMALL_MAX = SMALL_T * SMALL_ITEMS;
+constexpr uint32_t MASK_DEG = 32;      // manifolds of a body from which its colours are kept as a mask in memory
+constexpr uint16_t NO_COLOUR = 0xFFFFu;
+constexpr uint32_t SMALL_RANK = 96;    // contacts of a body up to which they are put in order by counting
+// shared memory: sort keys (then each manifold's places in its bodies' lists), priorities, wait counters, the lists,
+// colours, the rounds' queue, contact counts; the colour lists' buckets take the first four once the colours are known
+constexpr size_t SMALL_SMEM = SMALL_MAX * (8 + 4 + 4 + 4 + 2 + 2 + 1);
+struct SmallArgs {
+    uint32_t nc, nb, K, reduce, max_colors, mw, verify, cstride;
+    const uint32_t *L_a, *L_b, *cidx, *body_off;
+    const float4 *L_p, *L_n;
+    uint32_t *perm, *man_a, *man_b, *man_ca, *man_cb, *man_start, *man_count, *man_prio, *man_color;
+    uint32_t *bm_count, *masks;                     // per active body, set up here for those that need them
+    uint32_t *col_start, *col_list, *jds_off, *dev, *err;
+};
+
+// exclusive sum over the block's threads; *total gets the whole
+__device__ __forceinline__ uint32_t small_scan(uint32_t v, uint32_t *total) {
+    __shared__ uint32_t ws[SMALL_T / 32];
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= (uint32_t)o) x += y; }
+    if (lane == 31) ws[wid] = x;
+    __syncthreads();
+    if (wid == 0) {
+        uint32_t y = ws[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const uint32_t z = __shfl_up_sync(0xffffffffu, y, o); if (lane >= (uint32_t)o) y += z; }
+        ws[lane] = y;
+    }
+    __syncthreads();
+    const uint32_t before = (wid ? ws[wid - 1] : 0u) + x - v;
+    *total = ws[SMALL_T / 32 - 1];
+    __syncthreads();
+    return before;
+}
+// exclusive maximum over the block's threads before this one (0 for none)
+__device__ __forceinline__ uint32_t small_scan_max(uint32_t v) {
+    __shared__ uint32_t ws[SMALL_T / 32];
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= (uint32_t)o) x = max(x, y); }
+    if (lane == 31) ws[wid] = x;
+    __syncthreads();
+    uint32_t before = __shfl_up_sync(0xffffffffu, x, 1);
+    if (lane == 0) before = 0;
+    for (uint32_t w = 0; w < wid; w++) before = max(before, ws[w]);
+    __syncthreads();
+    return before;
+}
+// ascending bitonic sort of n2 (a power of two) keys
+__device__ __forceinline__ void small_sort(unsigned long long *key, uint32_t n2) {
+    for (uint32_t k = 2; k <= n2; k <<= 1)
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            for (uint32_t q = threadIdx.x; q < n2 / 2; q += SMALL_T) {
+                const uint32_t t = 2 * q - (q & (j - 1)), u = t + j;   // the q-th pair j apart
+                const unsigned long long x = key[t], y = key[u];
+                if ((x > y) == ((t & k) == 0)) { key[t] = y; key[u] = x; }
+            }
+            __syncthreads();
+        }
+}
+
+__global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
+    extern __shared__ __align__(16) unsigned char ss[];
+    unsigned long long *key = (unsigned long long *)ss;
+    uint32_t *prio = (uint32_t *)(ss + SMALL_MAX * 8), *wait = prio + SMALL_MAX;
+    uint16_t *list = (uint16_t *)(wait + SMALL_MAX), *colour = list + 2 * SMALL_MAX;
+    uint16_t *queue = colour + SMALL_MAX;
+    uint8_t *count = (uint8_t *)(queue + SMALL_MAX);
+    __shared__ uint32_t s_n, s_big, s_ncol, s_queue;
+    const uint32_t tid = threadIdx.x;
+    if (tid == 0) { s_n = 0; s_big = 0; s_ncol = 0; s_queue = 0; }
+    uint32_t nc = A.nc, items = (nc + SMALL_T - 1) / SMALL_T, t0 = tid * items;
+    {
+        uint32_t la[SMALL_ITEMS], lb[SMALL_ITEMS];
+#pragma unroll
+        for (int k = 0; k < SMALL_ITEMS; k++) {
+            const uint32_t t = tid + k * SMALL_T;
+            la[k] = t < nc ? A.L_a[t] : 0u;
+            lb[k] = t < nc ? A.L_b[t] : STATIC;
+        }
+#pragma unroll
+        for (int k = 0; k < SMALL_ITEMS; k++) {
+            const uint32_t t = tid + k * SMALL_T;
+            if (t < nc)
+                key[t] = ((unsigned long long)A.cidx[la[k]] << 30) |
+                         ((unsigned long long)(lb[k] == STATIC ? 0u : A.cidx[lb[k]] + 1) << 13) | t;
+        }
+    }
+    __syncthreads();
+    // each thread's run of contacts, t0 .. t0 + items, and where the body (drop = 30) or pair (13) of each begins
+    uint32_t begin[SMALL_ITEMS];
+    auto begins = [&](int drop) {
+        uint32_t own = 0;                           // the last place in the run where one begins, + 1
+#pragma unroll
+        for (int k = 0; k < SMALL_ITEMS; k++) {
+            const uint32_t t = t0 + k;
+            if (k < (int)items && t < nc && (t == 0 || (key[t] >> drop) != (key[t - 1] >> drop))) own = t + 1;
+            begin[k] = own;
+        }
+        const uint32_t last = small_scan_max(own);
+#pragma unroll
+        for (int k = 0; k < SMALL_ITEMS; k++) begin[k] = max(begin[k], last) - 1;
+    };
+    // Contacts by (a, b), each pair's in list order. The list comes in the bricks' order and a body's bricks lie together,
+    // so as a rule it only has to be put in order within each body: a contact's place is the number of smaller keys among
+    // its body's. A body with many contacts, or bodies out of order, take the whole sort.
+    begins(30);
+    {
+        unsigned long long own[SMALL_ITEMS];
+        uint32_t to[SMALL_ITEMS];
+        bool bad = false;
+#pragma unroll
+        for (int k = 0; k < SMALL_ITEMS; k++) {
+            const uint32_t t = t0 + k;
+            if (k >= (int)items || t >= nc) continue;
+            own[k] = key[t];
+            if (t && (key[t - 1] >> 30) > (own[k] >> 30)) bad = true;
+            // four at a time, past the body's end too (a larger body's keys are not smaller)
+            const unsigned long long body_end = ((own[k] >> 30) + 1) << 30;
+            uint32_t u = begin[k], less = 0;
+            for (bool more = true; more && u < begin[k] + SMALL_RANK; u += 4) {
+                unsigned long long x[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) x[e] = u + e < nc ? key[u + e] : ~0ull;
+#pragma unroll
+                for (int e = 0; e < 4; e++) less += x[e] < own[k] ? 1u : 0u;
+                more = x[3] < body_end;
+                if (more && u + 4 >= begin[k] + SMALL_RANK) bad = true;
+            }
+            to[k] = begin[k] + less;
+        }
+        if (__syncthreads_or(bad)) {
+            uint32_t n2 = 2;
+            while (n2 < nc) n2 <<= 1;
+            for (uint32_t t = nc + tid; t < n2; t += SMALL_T) key[t] = ~0ull;
+            __syncthreads();
+            small_sort(key, n2);
+        } else {
+#pragma unroll
+            for (int k = 0; k < SMALL_ITEMS; k++)
+                if (k < (int)items && t0 + k < nc) key[to[k]] = own[k];
+            __syncthreads();
+        }
+    }
+    begins(13);
+    if (A.reduce) {
+        // contact reduction (see RED_K above): a pair's contacts counted at its first place, which `first` gives
+        uint16_t *first = colour;
+        for (uint32_t t = tid; t < nc; t += SMALL_T) wait[t] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < SMALL_ITEMS; k++)
+            if (k < (int)items && t0 + k < nc) {
+                first[t0 + k] = (uint16_t)begin[k];
+                atomicAdd(&wait[begin[k]], 1u);
+            }
+        __syncthreads();
+        for (uint32_t t = tid; t < nc; t += SMALL_T)
+            if (first[t] == t) list[t] = wait[t] > RED_K ? (uint16_t)(atomicAdd(&s_big, 1u) + 1) : (uint16_t)0;
+        __syncthreads();
+        const uint32_t nbig = s_big;
+        if (nbig) {
+            // best score and winner per big pair and direction (at most 8192 / 33 pairs)
+            uint32_t *best = prio, *win = wait;
+            for (uint32_t t = tid; t < nbig * RED_S; t += SMALL_T) { best[t] = 0; win[t] = 0; }
+            __syncthreads();
+            auto each = [&](auto &&f) {
+                for (uint32_t t = tid; t < nc; t += SMALL_T) {
+                    const uint32_t g = list[first[t]];
+                    if (!g) continue;
+                    const uint32_t c = (uint32_t)key[t] & (SMALL_MAX - 1), o = (g - 1u) * RED_S;
+                    const float4 p = A.L_p[c];
+                    const float depth = A.L_n[c].w;
+                    // (each contact starts at another direction: a pair's share 27 words)
+                    for (uint32_t e = 0, d = c % RED_S; e < RED_S; e++, d = d + 1 == RED_S ? 0 : d + 1) f(o + d, f2o(red_score(p, depth, d)), c);
+                }
+                __syncthreads();
+            };
+            each([&](uint32_t o, uint32_t x, uint32_t) { if (x > *(volatile uint32_t *)&best[o]) atomicMax(&best[o], x); });
+            each([&](uint32_t o, uint32_t x, uint32_t c) { if (x == best[o]) atomicMax(&win[o], c + 1); });
+            unsigned long long kept[SMALL_ITEMS];
+            uint32_t mine = 0;
+#pragma unroll
+            for (int k = 0; k < SMALL_ITEMS; k++) {
+                kept[k] = ~0ull;
+                if (k >= (int)items || t0 + k >= nc) continue;
+                const uint32_t c = (uint32_t)key[t0 + k] & (SMALL_MAX - 1), g = list[begin[k]];
+                bool on = g == 0;
+                for (uint32_t d = 0; g && d < RED_S; d++) on |= win[(g - 1u) * RED_S + d] == c + 1;
+                if (on) { kept[k] = key[t0 + k]; mine++; }
+            }
+            uint32_t all, at = small_scan(mine, &all);
+#pragma unroll
+            for (int k = 0; k < SMALL_ITEMS; k++) if (kept[k] != ~0ull) key[at++] = kept[k];
+            nc = all;
+            items = (nc + SMALL_T - 1) / SMALL_T;
+            t0 = tid * items;
+            __syncthreads();
+            begins(13);
+        }
+    }
+    // chunks of K: the manifolds, in (a, b) order; each one's first contact, then its words
+    uint32_t mine = 0, nm;
+#pragma unroll
+    for (int k = 0; k < SMALL_ITEMS; k++)
+        if (k < (int)items && t0 + k < nc && (t0 + k - begin[k]) % A.K == 0) mine++;
+    uint32_t m = small_scan(mine, &nm);
+    uint16_t *head = list, *nth = colour;           // (neither is in use yet)
+#pragma unroll
+    for (int k = 0; k < SMALL_ITEMS; k++) {
+        const uint32_t t = t0 + k;
+        if (k >= (int)items || t >= nc) continue;
+        A.perm[t] = (uint32_t)key[t] & (SMALL_MAX - 1);
+        if ((t - begin[k]) % A.K) continue;
+        head[m] = (uint16_t)t;
+        nth[m++] = (uint16_t)((t - begin[k]) / A.K);
+    }
+    // per active body a word: its manifolds (low half), then the start of their list (high half)
+    uint32_t *body = A.nb <= SMALL_MAX ? wait : A.bm_count;
+    if (A.nb <= SMALL_MAX)
+        for (uint32_t q = tid; q < A.nb; q += SMALL_T) body[q] = 0;
+    __syncthreads();
+    uint32_t ca[SMALL_ITEMS], cb[SMALL_ITEMS];      // of this thread's manifolds tid + k SMALL_T
+#pragma unroll
+    for (int k = 0; k < SMALL_ITEMS; k++) {
+        const uint32_t q = tid + k * SMALL_T;
+        ca[k] = 0;
+        cb[k] = STATIC;
+        if (q >= nm) continue;
+        const uint32_t t = head[q], c = (uint32_t)key[t] & (SMALL_MAX - 1), j = nth[q];
+        const uint32_t n = (q + 1 < nm ? (uint32_t)head[q + 1] : nc) - t;
+        const uint32_t a = A.L_a[c], b = A.L_b[c], off = A.body_off[a];
+        const uint32_t h = pair_priority(a - off, b == STATIC ? 0u : b - off + 1u);
+        const uint32_t pr = j ? pair_priority(h, j) : h;
+        ca[k] = (uint32_t)(key[t] >> 30);
+        if (b != STATIC) cb[k] = (uint32_t)(key[t] >> 13 & 0x1FFFFu) - 1u;
+        A.man_a[q] = a; A.man_b[q] = b; A.man_ca[q] = ca[k]; A.man_cb[q] = cb[k];
+        A.man_start[q] = t; A.man_count[q] = n; A.man_prio[q] = pr;
+        prio[q] = pr;
+        count[q] = (uint8_t)n;
+        if (A.nb > SMALL_MAX) {
+            body[ca[k]] = 0;
+            if (b != STATIC) body[cb[k]] = 0;
+        }
+    }
+    __syncthreads();
+    // the bodies' manifold lists: counted, given their places, filled
+    uint16_t *pl = (uint16_t *)key;                 // per manifold: start and length of its first, then second body's list
+#pragma unroll
+    for (int k = 0; k < SMALL_ITEMS; k++) {
+        const uint32_t q = tid + k * SMALL_T;
+        if (q >= nm) continue;
+        pl[4 * q] = (uint16_t)(atomicAdd(&body[ca[k]], 1u) & 0xFFFFu);
+        pl[4 * q + 2] = cb[k] == STATIC ? 0 : (uint16_t)(atomicAdd(&body[cb[k]], 1u) & 0xFFFFu);
+        colour[q] = NO_COLOUR;
+    }
+    __syncthreads();
+    auto word = [&](uint32_t c) { return A.nb <= SMALL_MAX ? body[c] : __ldcg(&body[c]); };
+#pragma unroll
+    for (int k = 0; k < SMALL_ITEMS; k++) {
+        const uint32_t q = tid + k * SMALL_T;
+        if (q >= nm) continue;
+        auto place = [&](uint32_t c) {
+            const uint32_t n = word(c) & 0xFFFFu;
+            atomicAdd(&body[c], atomicAdd(&s_n, n) << 16);
+            if (n > MASK_DEG)                       // many manifolds at one body: its colours are kept as a mask
+                for (uint32_t i = 0; i < A.mw; i++) A.masks[(size_t)c * A.mw + i] = 0;
+        };
+        if (pl[4 * q] == 0) place(ca[k]);
+        if (cb[k] != STATIC && pl[4 * q + 2] == 0) place(cb[k]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < SMALL_ITEMS; k++) {
+        const uint32_t q = tid + k * SMALL_T;
+        if (q >= nm) continue;
+        const uint32_t wa = word(ca[k]), wb = cb[k] == STATIC ? 0u : word(cb[k]);
+        list[(wa >> 16) + pl[4 * q]] = (uint16_t)q;
+        if (cb[k] != STATIC) list[(wb >> 16) + pl[4 * q + 2]] = (uint16_t)q;
+        pl[4 * q] = (uint16_t)(wa >> 16); pl[4 * q + 1] = (uint16_t)wa;
+        pl[4 * q + 2] = (uint16_t)(wb >> 16); pl[4 * q + 3] = (uint16_t)wb;
+    }
+    __syncthreads();
+    // a manifold waits for the conflicting ones of higher priority (ties to the lower index)
+    auto before = [&](uint32_t x, uint32_t y) { return prio[x] > prio[y] || (prio[x] == prio[y] && x < y); };
+    // the conflicting manifolds of q that `pick` takes, their list entries and words read four at a time
+    auto conflicts = [&](uint32_t q, auto &&pick_fn, auto &&f) {
+        for (int side = 0; side < 2; side++) {
+            const uint32_t s0 = pl[4 * q + 2 * side], n = pl[4 * q + 2 * side + 1];
+            for (uint32_t k = 0; k < n; k += 4) {
+                uint32_t x[4];
+                bool on[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) x[e] = k + e < n ? list[s0 + k + e] : q;
+#pragma unroll
+                for (int e = 0; e < 4; e++) on[e] = x[e] != q && pick_fn(x[e]);
+#pragma unroll
+                for (int e = 0; e < 4; e++) if (on[e]) f(x[e]);
+            }
+        }
+    };
+    // the smallest colour free at both bodies: from the lists' coloured manifolds, or the masks of bodies that keep one
+    auto paint = [&](uint32_t q) {
+        const uint32_t sa = pl[4 * q], na = pl[4 * q + 1], sb = pl[4 * q + 2], nb = pl[4 * q + 3];
+        const uint32_t a = na > MASK_DEG ? A.man_ca[q] : 0u, b = nb > MASK_DEG ? A.man_cb[q] : 0u;
+        uint32_t c = 0xFFFFFFFFu;
+        for (uint32_t k = 0; k < A.mw && c == 0xFFFFFFFFu; k++) {
+            uint32_t used = 0;
+            auto gather = [&](uint32_t s0, uint32_t n, uint32_t body_id) {
+                if (n > MASK_DEG) { used |= __ldcg(&A.masks[(size_t)body_id * A.mw + k]); return; }
+                for (uint32_t i = 0; i < n; i += 4) {
+                    uint32_t x[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) x[e] = i + e < n ? list[s0 + i + e] : q;   // (q has no colour yet)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) x[e] = colour[x[e]];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) if (x[e] >> 5 == k) used |= 1u << (x[e] & 31u);
+                }
+            };
+            gather(sa, na, a);
+            gather(sb, nb, b);
+            if (~used) c = 32 * k + (__ffs(~used) - 1);
+        }
+        if (c >= A.max_colors) { atomicOr(A.err, (unsigned)ERR_CAPACITY_COLORS); c = A.max_colors - 1; }
+        if (na > MASK_DEG) atomicOr(&A.masks[(size_t)a * A.mw + (c >> 5)], 1u << (c & 31));
+        if (nb > MASK_DEG) atomicOr(&A.masks[(size_t)b * A.mw + (c >> 5)], 1u << (c & 31));
+        return c;
+    };
+    // rounds over a queue: the manifolds that wait for none, then those whose last one was coloured in the round before (few
+    // warps have work in a round, and the others only meet at its barriers)
+    for (uint32_t q = tid; q < nm; q += SMALL_T) {
+        uint32_t n = 0;
+        conflicts(q, [&](uint32_t x) { return before(x, q); }, [&](uint32_t) { n++; });
+        wait[q] = n;
+        if (n == 0) queue[atomicAdd(&s_queue, 1u)] = (uint16_t)q;
+    }
+    __syncthreads();
+    uint32_t rounds = 0, most = 0;
+    for (uint32_t lo = 0, hi = s_queue; lo < hi; rounds++) {
+        __syncthreads();
+        for (uint32_t i = lo + tid; i < hi; i += SMALL_T) {
+            const uint32_t q = queue[i], c = paint(q);   // (no conflicting manifold is in the same round)
+            colour[q] = (uint16_t)c;
+            most = max(most, c + 1);
+            for (int side = 0; side < 2; side++) {   // (as conflicts, with the four counters' atomics in flight together)
+                const uint32_t s0 = pl[4 * q + 2 * side], n = pl[4 * q + 2 * side + 1];
+                for (uint32_t k = 0; k < n; k += 4) {
+                    uint32_t x[4], old[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) x[e] = k + e < n ? list[s0 + k + e] : q;
+#pragma unroll
+                    for (int e = 0; e < 4; e++) old[e] = x[e] != q && before(q, x[e]) ? atomicSub(&wait[x[e]], 1u) : 0u;
+#pragma unroll
+                    for (int e = 0; e < 4; e++) if (old[e] == 1u) queue[atomicAdd(&s_queue, 1u)] = (uint16_t)x[e];
+                }
+            }
+        }
+        __syncthreads();
+        lo = hi;
+        hi = s_queue;
+    }
+    atomicMax(&s_ncol, most);
+    if (A.verify)
+        for (uint32_t q = tid; q < nm; q += SMALL_T)
+            conflicts(q, [&](uint32_t x) { return colour[x] == colour[q]; }, [&](uint32_t) { atomicOr(A.err, (unsigned)ERR_VERIFY_COLOR); });
+    __syncthreads();
+    // colour lists: buckets (colour, contact count descending), then each colour's start and the contact layout
+    const uint32_t ncol = s_ncol, nb = ncol * JDS_ROW;
+    uint32_t *hist = (uint32_t *)ss;
+    for (uint32_t q = tid; q < nb; q += SMALL_T) hist[q] = 0;
+    __syncthreads();
+    for (uint32_t q = tid; q < nm; q += SMALL_T) {
+        A.man_color[q] = colour[q];
+        atomicAdd(&hist[colour[q] * JDS_ROW + (JDS_K - count[q])], 1u);
+    }
+    __syncthreads();
+    uint32_t total = 0, n[JDS_K];                   // thread c: colour c's contacts, and its manifolds with more than k
+    if (tid < ncol) {
+        uint32_t run = 0;
+#pragma unroll
+        for (int j = 0; j < JDS_K; j++) { run += hist[tid * JDS_ROW + j]; n[JDS_K - 1 - j] = run; total += run; }
+    }
+    uint32_t whole, base = small_scan(total, &whole);
+    if (tid < ncol) {
+#pragma unroll
+        for (int k = 0; k < JDS_K; k++) { A.jds_off[tid * JDS_K + k] = base; base += n[k]; }
+    }
+    const uint32_t per = (nb + SMALL_T - 1) / SMALL_T;
+    uint32_t sum = 0;
+    for (uint32_t k = 0; k < per && tid * per + k < nb; k++) sum += hist[tid * per + k];
+    uint32_t run = small_scan(sum, &whole);
+    for (uint32_t k = 0; k < per && tid * per + k < nb; k++) { const uint32_t v = hist[tid * per + k]; hist[tid * per + k] = run; run += v; }
+    __syncthreads();
+    for (uint32_t c = tid; c <= A.cstride; c += SMALL_T) A.col_start[c] = c < ncol ? hist[c * JDS_ROW] : nm;
+    __syncthreads();
+    for (uint32_t q = tid; q < nm; q += SMALL_T) A.col_list[atomicAdd(&hist[colour[q] * JDS_ROW + (JDS_K - count[q])], 1u)] = q;
+    if (tid == 0) {
+        A.dev[DV_MANIFOLDS] = nm;
+        A.dev[DV_COLORS] = ncol;
+        A.dev[DV_ROUNDS] = rounds;
+        A.dev[DV_KEPT] = nc;
+    }
+}
+
 // ---------------------------------------------------------------- the coloured sequential-impulse solve
 // Contact layout (jagged diagonal, per colour): a colour's manifolds are listed by contact count, most first, and
 // contact k of the colour's p-th manifold sits at jds_off[colour * JDS_K + k] + p. The k-th contacts of a colour's
@@ -1530,7 +1947,7 @@ __device__ __forceinline__ void cp_async16(float4 *to, const float4 *from) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from) : "memory");
 }
 template <int NB, int T>
-__global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, uint32_t nc, uint32_t slots) {
+__global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *nc_p, uint32_t slots) {
     extern __shared__ float4 sv[];                 // velocity, spin of bodies rank, rank + NB, ...; then the contacts
     __shared__ uint32_t s_start[SOLVE_TEAM_COLS + 1], s_off[SOLVE_TEAM_COLS * JDS_K + 1], s_loc[SOLVE_TEAM_COLS * JDS_K + 1];
     __shared__ uint32_t s_base[NB];                // shared::cluster address of every block's velocities
@@ -1544,7 +1961,7 @@ __global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, uint32_t nc, uint
     uint32_t used = 0;
     if (tab) {
         for (uint32_t k = threadIdx.x; k <= ncol; k += T) s_start[k] = A.col_start[k];
-        for (uint32_t k = threadIdx.x; k <= rows; k += T) s_off[k] = k < rows ? A.jds_off[k] : nc;
+        for (uint32_t k = threadIdx.x; k <= rows; k += T) s_off[k] = k < rows ? A.jds_off[k] : *nc_p;
         __syncthreads();
         // row (colour, k): the k-th contacts of the colour's manifolds, n of them; those of this block are positions
         // rank, rank + NB, ... and go to consecutive slots
@@ -2042,6 +2459,7 @@ sf_status step_create(sf_world *w) {
     SF_CUDA(S->bucket_bits.alloc((size_t)nsc * (HSIZE / 32)));
     SF_CUDA(S->scene_awake.alloc(nsc)); SF_CUDA(S->scene_bricks.alloc(nsc));
     SF_CUDA(S->bstart.alloc((size_t)nsc * HSIZE + 1)); SF_CUDA(S->bsig.alloc((size_t)nsc * (HSIZE / 2)));
+    SF_CUDA(cudaFuncSetAttribute(k_small_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_SMEM));
     SF_CUDA(cudaFuncSetAttribute(k_contacts_gen_tab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEN_TAB_SMEM));
     SF_CUDA(S->srec.alloc(nd)); SF_CUDA(S->sent.alloc(nd));
     SF_CUDA(S->slot_id.alloc((size_t)nd * CSLOTS)); SF_CUDA(S->slot_p.alloc((size_t)nd * CSLOTS)); SF_CUDA(S->slot_n.alloc((size_t)nd * CSLOTS));
@@ -2078,6 +2496,7 @@ sf_status step_create(sf_world *w) {
     if (nb) SF_CUDA(cudaMemcpyAsync(S->body_off_of_body.p, off.data(), nb * 4, cudaMemcpyHostToDevice, s));
     uint64_t initial = w->P.contact_capacity ? w->P.contact_capacity : (uint64_t)std::max<uint32_t>(nd, 1) * 4;
     SF_CUDA(grow_contacts(S, initial));
+    SF_CUDA(S->M_id.alloc(std::min<uint64_t>(S->capacity, nd))); SF_CUDA(S->M_k.alloc(5 * S->M_id.n));
     int occ = 0;
     {
         auto *one = k_solve_team<1, SOLVE_TEAM_T1>;
@@ -2367,7 +2786,7 @@ static sf_status substep(sf_world *w, float h) {
     unsigned per_sm = w->P.solve_blocks ? std::min<unsigned>(w->P.solve_blocks, top_occ)
                                         : (unsigned)S->solve_t.choose(sb, sci);
     if (one_block) sci = -1;
-    // A small substep (at most SMALL_SUBSTEP_CONTACTS contacts) colours on one block, whose rounds end at
+    // A small substep that the one-block build does not take (SMALL_SUBSTEP_CONTACTS contacts at most) colours on one block, whose rounds end at
     // __syncthreads instead of a grid barrier: a body with many chunks (a large piece on the ground) needs a round per
     // colour, and the rounds, not the work, set the time.
     const unsigned R = (one_block && nc <= SMALL_SUBSTEP_CONTACTS)
@@ -2377,7 +2796,23 @@ static sf_status substep(sf_world *w, float h) {
     const uint32_t cstride = w->P.max_colors;
     uint32_t ncm = nc;   // the contacts that enter the manifolds (fewer after a contact reduction)
     // manifolds
-    if (nc) {
+    const uint32_t mw = (w->P.max_colors + 31) / 32;
+    const bool small = one_block && nc <= SMALL_MAX && n_loose == 0;
+    uint32_t nseg = cstride;                 // (domain, colour) segments
+    if (nc && small) {
+        SmallArgs B;
+        B.nc = nc; B.nb = nb; B.K = w->P.manifold_chunk; B.reduce = w->P.reduce; B.max_colors = w->P.max_colors; B.mw = mw;
+        B.verify = w->P.verify; B.cstride = cstride; B.L_a = S->L_a.p; B.L_b = S->L_b.p; B.cidx = S->cidx.p;
+        B.body_off = S->body_off_of_body.p; B.L_p = S->L_p.p; B.L_n = S->L_n.p; B.perm = S->perm.p;
+        B.man_a = S->man_a.p; B.man_b = S->man_b.p; B.man_ca = S->man_ca.p; B.man_cb = S->man_cb.p;
+        B.man_start = S->man_start.p; B.man_count = S->man_count.p; B.man_prio = S->man_prio.p; B.man_color = S->man_color.p;
+        B.bm_count = S->bm_count.p; B.masks = S->masks.p; B.col_start = S->col_start.p;
+        B.col_list = S->col_list.p; B.jds_off = S->jds_off.p; B.dev = S->dev.p; B.err = w->err.p;
+        prof_mark(w);
+        k_small_build<<<1, SMALL_T, SMALL_SMEM, s>>>(B);
+        L++;
+        prof_mark(w);
+    } else if (nc) {
         sf_status pst = use_partition(w, R, one_block);
         if (pst != SF_OK) return pst;
         const uint32_t D = S->part_D;
@@ -2431,6 +2866,7 @@ static sf_status substep(sf_world *w, float h) {
             k_pair_start<<<g_nc, 256, 0, s>>>(ncm, S->mflag.p, S->mpos.p, S->pair_start.p);
             L += 8;
         }
+        if (one_block && ncm == nc) SF_CUDA(cudaMemcpyAsync(S->dev.p + DV_KEPT, S->dev.p + DV_CONTACTS, 4, cudaMemcpyDeviceToDevice, s));
         k_chunk_flags<<<g_nc, 256, 0, s>>>(ncm, K, S->mflag.p, S->mpos.p, S->pair_start.p, S->cflag.p);
         SF_CUDA(exclusive_scan_u32(S->cflag.p, S->cpos.p, ncm, S->dev.p + DV_MANIFOLDS, S->wk, s));
         k_man_write<<<g_nc, 256, 0, s>>>(ncm, K, S->cflag.p, S->cpos.p, S->mflag.p, S->mpos.p, S->pair_start.p, S->perm.p,
@@ -2446,7 +2882,6 @@ static sf_status substep(sf_world *w, float h) {
         // colouring, on the active list's body ids, each domain on its own blocks
         SF_CUDA(cudaMemsetAsync(S->bm_count.p, 0, ((size_t)nb + 1) * 4, s));
         SF_CUDA(cudaMemsetAsync(S->bm_fill.p, 0, ((size_t)nb + 1) * 4, s));
-        const uint32_t mw = (w->P.max_colors + 31) / 32;
         SF_CUDA(cudaMemsetAsync(S->masks.p, 0, (size_t)nb * mw * 4, s));
         SF_CUDA(cudaMemsetAsync(S->man_round.p, 0xFF, (size_t)nc * 4, s));
         k_bm_count<<<g_nc, 256, 0, s>>>(S->dev.p + DV_MANIFOLDS, S->man_ca.p, S->man_cb.p, S->bm_count.p,
@@ -2466,7 +2901,7 @@ static sf_status substep(sf_world *w, float h) {
         if (J.seq_launched) k_colour_seq<<<1, SEQ_T, 0, s>>>(J);
         SF_CUDA(cudaLaunchCooperativeKernel((void *)k_jp, dim3(R), dim3(SOLVE_BLOCK), jargs, 0, s));
         // colour lists: each (domain, colour) segment's manifolds by contact count (most first), and the contact layout
-        const uint32_t nseg = D * cstride;
+        nseg = D * cstride;
         SF_CUDA(cudaMemsetAsync(S->col_count.p, 0, (size_t)nseg * JDS_ROW * 4, s));
         SF_CUDA(cudaMemsetAsync(S->col_fill.p, 0, (size_t)nseg * JDS_ROW * 4, s));
         SF_CUDA(cudaMemsetAsync(S->dom_ncol.p, 0, (size_t)D * 4, s));
@@ -2487,6 +2922,8 @@ static sf_status substep(sf_world *w, float h) {
             L++;
         }
         prof_mark(w);
+    }
+    if (nc) {
         // the solve's records are sized by the manifolds that occur (at most a contact each), not by the contact capacity
         if (S->M_id.n < ncm) {
             const size_t want = std::min<size_t>(S->capacity, 2 * (size_t)ncm + 65536);
@@ -2539,7 +2976,7 @@ static sf_status substep(sf_world *w, float h) {
             const uint32_t want = alone ? ncm : ncm / SOLVE_TEAM_BLOCKS + SOLVE_TEAM_COLS * JDS_K;
             const uint32_t slots = std::min(want, (SOLVE_TEAM_SMEM - nbl * 32) / 96);
             const size_t smem = (size_t)nbl * 32 + (size_t)slots * 96;
-            if (alone) k_solve_team<1, SOLVE_TEAM_T1><<<1, SOLVE_TEAM_T1, smem, s>>>(A, ncm, slots);
+            if (alone) k_solve_team<1, SOLVE_TEAM_T1><<<1, SOLVE_TEAM_T1, smem, s>>>(A, S->dev.p + DV_KEPT, slots);
             else {
                 cudaLaunchConfig_t cfg = {};
                 cudaLaunchAttribute at[1];
@@ -2551,7 +2988,8 @@ static sf_status substep(sf_world *w, float h) {
                 cfg.stream = s;
                 cfg.attrs = at;
                 cfg.numAttrs = 1;
-                SF_CUDA(cudaLaunchKernelEx(&cfg, k_solve_team<SOLVE_TEAM_BLOCKS, SOLVE_TEAM_T>, A, ncm, slots));
+                SF_CUDA(cudaLaunchKernelEx(&cfg, k_solve_team<SOLVE_TEAM_BLOCKS, SOLVE_TEAM_T>, A,
+                                           (const uint32_t *)(S->dev.p + DV_KEPT), slots));
             }
         } else {
             SF_CUDA(cudaMemsetAsync(S->dom_gb.p, 0, (size_t)S->part_D * sizeof(GridBarrier), s));
