@@ -1,0 +1,35 @@
+"""The box world's teams at their edges, against the oracle bit for bit: one box, sizes around a warp, a block and the
+largest one-block scene, worlds of more scenes than SMs (two blocks of 256 threads an SM) and of fewer (one of 512).
+"""
+import numpy as np
+import pytest
+
+from shatterforge_b200 import boxes as X
+
+pytestmark = pytest.mark.gpu
+
+DT = np.float32(1.0 / 60.0)
+
+
+def check(oracle, scenes, params, steps):
+    w = X.BoxWorld(scenes, params)
+    ows = [oracle.OracleBoxWorld(s, params, oracle.ORDER_COLOR) for s in scenes]
+    for _ in range(steps):
+        w.step(DT)
+    for i, ow in enumerate(ows):
+        for _ in range(steps):
+            ow.step(DT)
+        st = w.stats(i)
+        assert st.status == 0
+        assert (st.awake, st.pairs, st.manifolds, st.points, st.colours) == ow.stats(), i
+        np.testing.assert_array_equal(w.state(i), ow.state())
+        np.testing.assert_array_equal(w.manifolds(i), ow.manifolds())
+
+
+@pytest.mark.parametrize("sizes", [
+    [1], [33, 1, 32, 31], [255, 256, 257], [511, 512, 513], [1023, 1025], [4096, 40], [4097, 255],
+    [20 + k % 23 for k in range(170)], [300 + k % 7 for k in range(150)],
+], ids=lambda s: f"{len(s)}x{max(s)}")
+def test_scene_sizes(sf, oracle, sizes):
+    steps = 6 if max(sizes) > 2000 else 12 if len(sizes) > 100 else 30
+    check(oracle, [X.pile(n) for n in sizes], X.box_params(allow_sleep=0, substeps=4), steps)
