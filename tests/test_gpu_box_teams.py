@@ -33,3 +33,22 @@ def check(oracle, scenes, params, steps):
 def test_scene_sizes(sf, oracle, sizes):
     steps = 6 if max(sizes) > 2000 else 12 if len(sizes) > 100 else 30
     check(oracle, [X.pile(n) for n in sizes], X.box_params(allow_sleep=0, substeps=4), steps)
+
+
+@pytest.mark.parametrize("under", [30, 34, 400, 1100])
+def test_pairs_of_one_body(sf, oracle, under):
+    """A static slab under `under` boxes: its list of pairs is sorted by its thread (up to 32), by the team, or (past the
+    980 that one walk keeps) walked for again."""
+    side = int(np.ceil(np.sqrt(under)))
+    k = np.arange(under)
+    recs = np.zeros((under + 1, 11), np.float32)
+    half = np.float32(0.14 * side)
+    recs[0] = [0, 0.5, 0, 0, 0, 0, 1, half, 0.5, half, 0.0]
+    recs[1:, 0] = (k % side - 0.5 * (side - 1)) * 0.28
+    recs[1:, 1] = 1.13
+    recs[1:, 2] = (k // side - 0.5 * (side - 1)) * 0.28
+    recs[1:, 6] = 1
+    recs[1:, 7:10] = 0.125
+    recs[1:, 10] = 1.0
+    recs[1:, :3] += np.random.default_rng(under).uniform(-0.004, 0.004, (under, 3)).astype(np.float32)
+    check(oracle, [recs, X.pile(40)], X.box_params(substeps=4), 20)
