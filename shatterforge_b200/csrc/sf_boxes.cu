@@ -61,8 +61,9 @@ struct BxArgs {
     int4 *ent_node;          // a grid entry's cell and the next entry of its hash slot
     uint32_t *cand_a, *cand_b, *hit; float *geom;
     DMan *man[2]; uint64_t *mkey[2]; uint32_t *mcount[2];
-    uint32_t *deg, *inc, *colour, *corder, *mwait;
-    uint64_t *mrank;
+    uint32_t *deg, *colour, *corder, *mwait;
+    uint2 *mnext;            // per manifold: the next lower priority on each of its bodies
+    ulonglong2 *cmask;       // per solver slot: the colours its manifolds took
     float4 *svw;             // per solver slot: velocity, spin
     float4 *sdt;             // per solver slot: the step's translation and rotation so far
     float4 *sol;             // the manifolds in colour order, BX_SC columns a scene (see SolMan)
@@ -738,10 +739,15 @@ __global__ void __launch_bounds__(T, CL == 1 && T <= 256 ? 2 : 1) k_box_step(BxA
     }
     team_sync<CL>();
     if (t == 0) { tm1 = gtime(); tns[1] += tm1 - tm0; tm0 = tm1; }
-    // ---- colouring: greedy in descending priority, by Jones-Plassmann rounds. A manifold takes the smallest colour
-    // its higher-priority neighbours (manifolds sharing a moving body) left free once all of them have one.
+    // ---- colouring: greedy in descending priority. A manifold takes the smallest colour that its higher-priority neighbours
+    // (manifolds sharing a moving body) left free once all of them have one: once it is the first uncoloured one of both its
+    // bodies, whose used colours are then a mask each. One pass over its bodies' lists, which hold the priorities themselves,
+    // tells a manifold whether a higher one is before it and which is the next lower one; a coloured manifold counts its two
+    // next ones down and goes on with one that became ready, the others are found by the next round.
+    // Rounds of polls that read every neighbour's priority and colour (17 of them, a barrier each) took 1.03 ms a step of 20,000
+    // boxes on a cluster, now 0.45 in 10 rounds, and 0.46 of 2,000 on a block, now 0.30.
     const uint32_t ns = n + 1;
-    for (uint32_t k = t; k < ns; k += TT) A.deg[s0 + k] = 0;
+    for (uint32_t k = t; k < ns; k += TT) { A.deg[s0 + k] = 0; A.cmask[s0 + k] = make_ulonglong2(0ull, 0ull); }
     for (uint32_t m = t; m < M; m += TT) A.colour[m0 + m] = BX_UNC;
     team_sync<CL>();
     for (uint32_t m = t; m < M; m += TT) {
@@ -751,32 +757,36 @@ __global__ void __launch_bounds__(T, CL == 1 && T <= 256 ? 2 : 1) k_box_step(BxA
     }
     team_sync<CL>();
     team_scan<T, CL>(A.deg + s0, ns, wsum, Gp + G_CTA, t, rank);
+    uint64_t *inc = (uint64_t *)(A.geom + (size_t)c0 * 20);      // 2 mcap words of 8 bytes, in the room of the contact geometry (980 n of 4)
     for (uint32_t m = t; m < M; m += TT) {
         const uint2 mm = A.mslot[m0 + m];
-        if (mm.x) A.inc[2 * (size_t)m0 + atomicAdd(&A.deg[s0 + mm.x], 1u)] = m;
-        if (mm.y) A.inc[2 * (size_t)m0 + atomicAdd(&A.deg[s0 + mm.y], 1u)] = m;
+        const uint64_t ab = A.mkey[par][m0 + m], rk = man_rank((uint32_t)(ab >> 32), (uint32_t)ab, m);
+        if (mm.x) inc[atomicAdd(&A.deg[s0 + mm.x], 1u)] = rk;
+        if (mm.y) inc[atomicAdd(&A.deg[s0 + mm.y], 1u)] = rk;
     }
     team_sync<CL>();
-    // incident list of slot k: [k ? deg[k - 1] : 0, deg[k]). Each manifold counts its higher-priority neighbours;
-    // a coloured manifold counts its lower-priority neighbours down, and one whose count reaches 0 takes its colour.
+    // list of slot k: [k ? deg[k - 1] : 0, deg[k])
     volatile uint32_t *col = A.colour + m0;
-    uint64_t *prio = A.mrank + m0;
     uint32_t *wait = A.mwait + m0;
-    for (uint32_t m = t; m < M; m += TT) { const uint64_t ab = A.mkey[par][m0 + m]; prio[m] = man_rank((uint32_t)(ab >> 32), (uint32_t)ab, m); }
-    team_sync<CL>();
     for (uint32_t m = t; m < M; m += TT) {
         const uint2 mm = A.mslot[m0 + m];
-        const uint64_t rk = prio[m];
-        uint32_t hi_n = 0;
+        const uint64_t ab = A.mkey[par][m0 + m], rk = man_rank((uint32_t)(ab >> 32), (uint32_t)ab, m);
+        uint32_t nx[2], before = 0;
         for (int side = 0; side < 2; side++) {
             const uint32_t sl = side ? mm.y : mm.x;
-            if (!sl) continue;
-            for (uint32_t q = A.deg[s0 + sl - 1], e = A.deg[s0 + sl]; q < e; q++) {
-                const uint32_t o = A.inc[2 * (size_t)m0 + q];
-                if (o != m && prio[o] > rk) hi_n++;
-            }
+            uint64_t lower = 0;
+            bool higher = false;
+            if (sl)
+                for (uint32_t q = A.deg[s0 + sl - 1], e = A.deg[s0 + sl]; q < e; q++) {
+                    const uint64_t o = inc[q];
+                    higher |= o > rk;
+                    if (o < rk && o > lower) lower = o;
+                }
+            before += higher;
+            nx[side] = lower ? 0xFFFFFFFFu - (uint32_t)lower : BX_UNC;      // (a priority's low word is ~m)
         }
-        wait[m] = hi_n;
+        wait[m] = before;
+        A.mnext[m0 + m] = make_uint2(nx[0], nx[1]);
     }
     team_sync<CL>();
     uint32_t rounds = 0;
@@ -784,32 +794,23 @@ __global__ void __launch_bounds__(T, CL == 1 && T <= 256 ? 2 : 1) k_box_step(BxA
         int pend = 0;
         for (uint32_t m = t; m < M; m += TT) {
             if (col[m] != BX_UNC) continue;
-            if (((volatile uint32_t *)wait)[m] != 0) { pend = 1; continue; }
-            if constexpr (CL == 1) __threadfence_block(); else __threadfence();
-            const uint2 mm = A.mslot[m0 + m];
-            const uint64_t rk = prio[m];
-            uint64_t used0 = 0, used1 = 0;
-            for (int side = 0; side < 2; side++) {
-                const uint32_t sl = side ? mm.y : mm.x;
-                if (!sl) continue;
-                for (uint32_t q = A.deg[s0 + sl - 1], e = A.deg[s0 + sl]; q < e; q++) {
-                    const uint32_t o = A.inc[2 * (size_t)m0 + q];
-                    if (o == m || prio[o] < rk) continue;
-                    const uint32_t oc = col[o];
-                    if (oc < 64) used0 |= 1ull << oc; else if (oc < 128) used1 |= 1ull << (oc - 64);
-                }
-            }
-            uint32_t c = ~used0 ? (uint32_t)__ffsll((long long)~used0) - 1 : (~used1 ? 64u + (uint32_t)__ffsll((long long)~used1) - 1 : (uint32_t)BX_MAXC);
-            if (c >= (uint32_t)BX_MAXC) { atomicOr(&Gp[G_ERR], (uint32_t)BXE_COLOURS); c = BX_MAXC - 1; }
-            col[m] = c;
-            if constexpr (CL == 1) __threadfence_block(); else __threadfence();
-            for (int side = 0; side < 2; side++) {
-                const uint32_t sl = side ? mm.y : mm.x;
-                if (!sl) continue;
-                for (uint32_t q = A.deg[s0 + sl - 1], e = A.deg[s0 + sl]; q < e; q++) {
-                    const uint32_t o = A.inc[2 * (size_t)m0 + q];
-                    if (o != m && prio[o] < rk) atomicSub(&wait[o], 1u);
-                }
+            if (((volatile uint32_t *)wait)[m] != 0 || atomicCAS(&wait[m], 0u, BX_UNC) != 0) { pend = 1; continue; }   // (claimed: BX_UNC)
+            for (uint32_t x = m; x != BX_UNC;) {
+                if constexpr (CL == 1) __threadfence_block(); else __threadfence();
+                const uint2 mm = A.mslot[m0 + x], nx = A.mnext[m0 + x];
+                volatile unsigned long long *ua = (volatile unsigned long long *)(A.cmask + s0 + mm.x), *ub = (volatile unsigned long long *)(A.cmask + s0 + mm.y);
+                const unsigned long long a0 = mm.x ? ua[0] : 0ull, a1 = mm.x ? ua[1] : 0ull, q0 = mm.y ? ub[0] : 0ull, q1 = mm.y ? ub[1] : 0ull;
+                const unsigned long long free0 = ~(a0 | q0), free1 = ~(a1 | q1);
+                uint32_t c = free0 ? (uint32_t)__ffsll((long long)free0) - 1 : (free1 ? 64u + (uint32_t)__ffsll((long long)free1) - 1 : (uint32_t)BX_MAXC);
+                if (c >= (uint32_t)BX_MAXC) { atomicOr(&Gp[G_ERR], (uint32_t)BXE_COLOURS); c = BX_MAXC - 1; }
+                const unsigned long long bit = 1ull << (c & 63u);
+                if (mm.x) { if (c < 64) ua[0] = a0 | bit; else ua[1] = a1 | bit; }
+                if (mm.y) { if (c < 64) ub[0] = q0 | bit; else ub[1] = q1 | bit; }
+                col[x] = c;
+                if constexpr (CL == 1) __threadfence_block(); else __threadfence();
+                x = BX_UNC;
+                if (nx.x != BX_UNC && atomicSub(&wait[nx.x], 1u) == 1 && atomicCAS(&wait[nx.x], 0u, BX_UNC) == 0) x = nx.x;
+                if (nx.y != BX_UNC && atomicSub(&wait[nx.y], 1u) == 1 && x == BX_UNC && atomicCAS(&wait[nx.y], 0u, BX_UNC) == 0) x = nx.y;
             }
         }
         rounds++;
@@ -967,15 +968,16 @@ struct sf_box_world {
     DBuf<DM3> rot, sii;
     DBuf<P3> sp0;
     DBuf<float4> alo, ahi, svw, sdt, sol;
-    DBuf<uint2> mslot;
+    DBuf<uint2> mslot, mnext;
     DBuf<float> sim, geom;
     DBuf<float4> sq;
-    DBuf<uint32_t> ecnt, sidx, cand_n, seglong, uf, mint, ent_body, head, cand_a, cand_b, hit, deg, inc, colour,
+    DBuf<uint32_t> ecnt, sidx, cand_n, seglong, uf, mint, ent_body, head, cand_a, cand_b, hit, deg, colour,
         corder, mwait, stats, mcount0, mcount1, sc_b0, sc_n, sc_e0, sc_t0, sc_tcap, sc_c0, sc_m0;
     DBuf<int4> ent_node;
     DBuf<uint8_t> wake;
     DBuf<DMan> man0, man1;
-    DBuf<uint64_t> mkey0, mkey1, mrank;
+    DBuf<uint64_t> mkey0, mkey1;
+    DBuf<ulonglong2> cmask;
     DBuf<unsigned long long> tns;
     DBuf<uint32_t> gs, slist;
     uint32_t n_small = 0, n_big = 0;
@@ -1060,7 +1062,7 @@ extern "C" sf_status sf_box_world_create(const float *boxes, const uint32_t *sce
     A(w->sim.alloc(ns)); A(w->sq.alloc(ns)); A(w->deg.alloc(ns));
     A(w->ent_body.alloc(et)); A(w->ent_node.alloc(et)); A(w->head.alloc(tt));
     A(w->cand_a.alloc(ct)); A(w->cand_b.alloc(ct)); A(w->hit.alloc(ct)); A(w->geom.alloc(20 * ct));
-    A(w->colour.alloc(mt)); A(w->corder.alloc(mt)); A(w->mwait.alloc(mt)); A(w->mrank.alloc(mt)); A(w->inc.alloc(2 * mt));
+    A(w->colour.alloc(mt)); A(w->corder.alloc(mt)); A(w->mwait.alloc(mt)); A(w->mnext.alloc(mt)); A(w->cmask.alloc(ns));
     A(w->man0.alloc(mt)); A(w->man1.alloc(mt)); A(w->mkey0.alloc(mt)); A(w->mkey1.alloc(mt));
     A(w->stats.alloc((size_t)n_scenes * 8)); A(w->tns.alloc((size_t)n_scenes * 5));
     A(w->gs.alloc((size_t)n_scenes * BX_G)); A(w->slist.alloc(n_scenes)); A(w->mcount0.alloc(n_scenes)); A(w->mcount1.alloc(n_scenes));
@@ -1127,7 +1129,7 @@ extern "C" sf_status sf_box_world_step(sf_box_world *w, float dt, uint32_t nstep
     a.cand_a = w->cand_a.p; a.cand_b = w->cand_b.p; a.hit = w->hit.p; a.geom = w->geom.p;
     a.man[0] = w->man0.p; a.man[1] = w->man1.p; a.mkey[0] = w->mkey0.p; a.mkey[1] = w->mkey1.p;
     a.mcount[0] = w->mcount0.p; a.mcount[1] = w->mcount1.p;
-    a.deg = w->deg.p; a.inc = w->inc.p; a.colour = w->colour.p; a.corder = w->corder.p; a.mwait = w->mwait.p; a.mrank = w->mrank.p;
+    a.deg = w->deg.p; a.colour = w->colour.p; a.corder = w->corder.p; a.mwait = w->mwait.p; a.mnext = w->mnext.p; a.cmask = w->cmask.p;
     a.svw = w->svw.p; a.sdt = w->sdt.p; a.sol = w->sol.p; a.mslot = w->mslot.p; a.sp0 = w->sp0.p; a.sim = w->sim.p; a.sii = w->sii.p;
     a.sq = w->sq.p;
     a.sc_b0 = w->sc_b0.p; a.sc_n = w->sc_n.p; a.sc_e0 = w->sc_e0.p; a.sc_t0 = w->sc_t0.p; a.sc_tcap = w->sc_tcap.p;

@@ -52,3 +52,38 @@ def test_pairs_of_one_body(sf, oracle, under):
     recs[1:, 10] = 1.0
     recs[1:, :3] += np.random.default_rng(under).uniform(-0.004, 0.004, (under, 3)).astype(np.float32)
     check(oracle, [recs, X.pile(40)], X.box_params(substeps=4), 20)
+
+
+@pytest.mark.parametrize("under", [1, 63, 70, 140])
+def test_colours_of_one_body(sf, oracle, under):
+    """A moving plate on `under` boxes: as many colours as it has manifolds, in one or two mask words, and past the 128
+    that there are the step is refused and the scene left as it was, while the other scene steps as its oracle."""
+    side = int(np.ceil(np.sqrt(under)))
+    k = np.arange(under)
+    recs = np.zeros((under + 1, 11), np.float32)
+    half = np.float32(0.14 * side)
+    recs[:under, 0] = (k % side - 0.5 * (side - 1)) * 0.28
+    recs[:under, 1] = 0.125
+    recs[:under, 2] = (k // side - 0.5 * (side - 1)) * 0.28
+    recs[:under, 7:10] = 0.125
+    recs[under, 1] = 0.255
+    recs[under, :3] += [0, 0.1, 0]
+    recs[under, 7:10] = [half, 0.1, half]
+    recs[:, 6] = 1
+    recs[:, 10] = 1.0
+    other = X.pile(40)
+    p = X.box_params(allow_sleep=0, substeps=4)
+    if under <= 128:
+        check(oracle, [recs, other], p, 20)
+        return
+    w = X.BoxWorld([recs, other], p)
+    before = w.state(0).copy()
+    ow = oracle.OracleBoxWorld(other, p, oracle.ORDER_COLOR)
+    for _ in range(3):
+        with pytest.raises(sf.SfError) as e:
+            w.step(DT)
+        assert e.value.status == sf.SF_ERR_CAPACITY
+        ow.step(DT)
+    assert w.stats(0).status == 8
+    np.testing.assert_array_equal(w.state(0), before)
+    np.testing.assert_array_equal(w.state(1), ow.state())
