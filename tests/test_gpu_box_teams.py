@@ -87,3 +87,19 @@ def test_colours_of_one_body(sf, oracle, under):
     assert w.stats(0).status == 8
     np.testing.assert_array_equal(w.state(0), before)
     np.testing.assert_array_equal(w.state(1), ow.state())
+
+
+def test_state_words(sf, oracle):
+    """The 22 floats of a box, for boxes asleep and awake, against the oracle's records; the state of a world that has not
+    stepped is its records."""
+    recs = X.pile(100)
+    w = X.BoxWorld([recs, X.stack(20)], X.box_params())
+    s = w.state(0)
+    np.testing.assert_array_equal(s[:, :7], recs[:, :7])
+    np.testing.assert_array_equal(s[:, 7:14], np.zeros((100, 7), np.float32))
+    ow = oracle.OracleBoxWorld(X.stack(20), X.box_params(), oracle.ORDER_COLOR)
+    for _ in range(90):
+        w.step(DT)
+        ow.step(DT)
+        np.testing.assert_array_equal(w.state(1), ow.state())
+    assert w.state(1)[:, 21].sum() in (0, 20) and w.state(1)[:, 13].max() >= 0.5
