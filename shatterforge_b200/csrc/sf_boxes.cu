@@ -37,6 +37,7 @@ constexpr uint32_t BX_EPB = 27;      // grid entries a body may take, on average
 constexpr uint32_t BX_CPB = 8;       // manifolds a body may take, on average over its scene
 constexpr int BX_MAXC = 128;         // colours
 constexpr uint32_t BX_BIG = 4096;    // scenes above this many boxes step on a thread-block cluster
+constexpr uint32_t BX_MID = 1024;    // and scenes above this many, where the whole world then runs as clusters side by side
 constexpr int BX_CL = 16, BX_CL_THREADS = 512;
 enum { BXE_ENTRIES = 1, BXE_PAIRS = 2, BXE_MANIFOLDS = 4, BXE_COLOURS = 8, BXE_GUARD = 16 };
 
@@ -1094,8 +1095,29 @@ extern "C" sf_status sf_box_world_create(const float *boxes, const uint32_t *sce
         delete w; set_error("upload failed"); return SF_ERR_CUDA;
     }
     {
+        uint32_t least = 0xFFFFFFFFu;
+        for (uint32_t s = 0; s < n_scenes; s++) least = std::min(least, w->nn[s]);
+        int ncl = 0;      // clusters the chip runs at once
+        if (w->max_n > BX_BIG || least > BX_MID) {
+            cudaFuncSetAttribute(k_box_step<BX_CL_THREADS, BX_CL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            cudaLaunchConfig_t c = {};
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = BX_CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+            c.gridDim = dim3(BX_CL);
+            c.blockDim = dim3(BX_CL_THREADS);
+            c.attrs = at;
+            c.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&ncl, k_box_step<BX_CL_THREADS, BX_CL>, &c) != cudaSuccess) { ncl = 0; cudaGetLastError(); }
+            w->cluster_ok = ncl > 0;
+        }
+        // A cluster's barriers cost what a block's longer loops do at some 1,000 boxes. Measured a pass of two steps of 12 (4)
+        // sub-steps, block against cluster: one scene of 700 boxes 2.3, 2.4 ms; 1,000 2.9, 2.7 (2.6, 1.8); 2,000 5.0, 3.0 (3.8,
+        // 1.7); 4,000 10.4, 3.9; but eight of 2,000, one more than fit at once, 5.5, 6.5. A world of fewer boxes in some
+        // scene keeps its one-block launch, which would run after the clusters.
+        const uint32_t line = least > BX_MID && n_scenes <= (uint32_t)ncl ? BX_MID : BX_BIG;
         std::vector<uint32_t> big, small;
-        for (uint32_t s = 0; s < n_scenes; s++) (w->nn[s] > BX_BIG ? big : small).push_back(s);
+        for (uint32_t s = 0; s < n_scenes; s++) (w->nn[s] > line ? big : small).push_back(s);
         w->n_big = (uint32_t)big.size(); w->n_small = (uint32_t)small.size();
         // One block an SM is enough for the scenes: 512 threads each, not two blocks of 256. Measured a pass of two steps:
         // 148 scenes of 2,000 boxes 11.3 against 15.1 ms, one of 2,000 6.9 against 9.9, but 300 of 300 5.7 against 4.5, and
@@ -1107,20 +1129,6 @@ extern "C" sf_status sf_box_world_create(const float *boxes, const uint32_t *sce
         if (w->n_small <= (uint32_t)sms && sn >= 256ull * w->n_small) w->small_t = 512;
         big.insert(big.end(), small.begin(), small.end());
         cudaMemcpy(w->slist.p, big.data(), n_scenes * 4, cudaMemcpyHostToDevice);
-        if (w->n_big) {
-            cudaFuncSetAttribute(k_box_step<BX_CL_THREADS, BX_CL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            cudaLaunchConfig_t c = {};
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = BX_CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-            c.gridDim = dim3(BX_CL);
-            c.blockDim = dim3(BX_CL_THREADS);
-            c.attrs = at;
-            c.numAttrs = 1;
-            int ncl = 0;
-            if (cudaOccupancyMaxActiveClusters(&ncl, k_box_step<BX_CL_THREADS, BX_CL>, &c) != cudaSuccess) { ncl = 0; cudaGetLastError(); }
-            w->cluster_ok = ncl > 0;
-        }
     }
     sf_status r = box_upload(w, boxes);
     if (r != SF_OK) { delete w; return r; }
@@ -1148,7 +1156,7 @@ extern "C" sf_status sf_box_world_step(sf_box_world *w, float dt, uint32_t nstep
     SF_CUDA(cudaMemsetAsync(w->tns.p, 0, (size_t)w->n_scenes * 5 * sizeof(unsigned long long), w->stream));
     SF_CUDA(cudaEventRecord(w->ev0, w->stream));
     for (uint32_t k = 0; k < nsteps; k++) {
-        // scenes of more than BX_BIG boxes: one 16-block cluster each; the rest: one block each
+        // the scenes past the line drawn at creation: one 16-block cluster each; the rest: one block each
         if (w->n_big && w->cluster_ok) {
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute at[1];

@@ -35,6 +35,13 @@ def test_scene_sizes(sf, oracle, sizes):
     check(oracle, [X.pile(n) for n in sizes], X.box_params(allow_sleep=0, substeps=4), steps)
 
 
+@pytest.mark.parametrize("sizes", [[1024], [1025], [1025] * 7, [1025] * 9, [1025, 4097], [1024, 4097]],
+                         ids=lambda s: "-".join(map(str, s)))
+def test_scenes_on_clusters_side_by_side(sf, oracle, sizes):
+    """Middling scenes take a cluster each where the whole world fits as clusters, else a block each."""
+    check(oracle, [X.pile(n) for n in sizes], X.box_params(allow_sleep=0, substeps=4), 8)
+
+
 @pytest.mark.parametrize("under", [30, 34, 400, 1100])
 def test_pairs_of_one_body(sf, oracle, under):
     """A static slab under `under` boxes: its list of pairs is sorted by its thread (up to 32), by the team, or (past the
