@@ -3,13 +3,13 @@
 // push_manifold with its warm start and friction anchors (phys.rs:447-497), the soft-step sub-steps (warm start,
 // biased solve, integrate, relax; phys.rs:216-324) and island sleep (phys.rs:326-354).
 //
-// One thread block runs one scene's whole step; a launch steps every scene of the world. Inside a scene:
+// One thread block, or one cluster, runs one scene's whole step; a launch steps every scene of its kind. Inside a scene:
 //   * the grid is a hash table of cell lists (linked entries, one per body and covered cell); the pair set is the
 //     reference's (AABB overlap, reported in the cell of the larger minimum corner);
 //   * every body lists its pairs with higher-numbered bodies, sorted, then its ground contact, so the manifold list
 //     comes out in key order (a, b; ground as b = NONE) with no global sort, and the previous step's manifolds are
 //     found by binary search in that order;
-//   * manifolds are coloured greedily in a fixed priority order (Jones-Plassmann rounds reach the same colouring),
+//   * manifolds are coloured greedily in a fixed priority order, each once it is the first left at both its bodies,
 //     and each solve pass runs colour by colour with a block barrier between colours: inside a colour no two
 //     manifolds share a moving body, so the result does not depend on the thread schedule;
 //   * sleeping islands come from a lock-free union-find over the manifolds between two moving bodies.

@@ -16,10 +16,11 @@
 //   colouring        Jones-Plassmann rounds on the manifold conflict graph (two manifolds conflict when they share
 //                    an awake body); priority = hash of the pair, ties to the lower manifold index; the smallest
 //                    colour free at both bodies — the same colouring as a greedy pass in priority order
+//   k_small_build    manifolds, colours and solve layout of a small substep (at most 8,192 contacts) in one block
 //   k_solve          persistent kernel: for each iteration, for each colour, each manifold's contacts solved in list
 //                    order with solve()'s sequential-impulse math (src/lib.rs:1579-1601); a bounded grid barrier
 //                    separates colours. Manifolds of one colour share no awake body, so the result does not
-//                    depend on their order inside a colour.
+//                    depend on their order inside a colour. Small substeps: k_solve_team, in shared memory.
 //   islands          union-find over manifolds between two awake bodies, larger root linked under the smaller by
 //                    CAS with path halving (gpu/gpu_world.js:1634-1655, engine/src/phys.rs:326-354)
 //   k_integrate      pinch clamps (src/lib.rs:1746-1768) and integrate (src/lib.rs:1703-1742)
