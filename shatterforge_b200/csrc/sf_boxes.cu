@@ -120,6 +120,9 @@ __device__ __forceinline__ void btangents(P3 n, P3 &t1, P3 &t2) {   // phys.rs:5
 }
 __device__ __forceinline__ float bfloor(float x) { float t = (float)(int32_t)x; return t > x ? t - 1.0f : t; }
 __device__ __forceinline__ int32_t bcell(float x, float inv_cell) { return (int32_t)bfloor(x * inv_cell); }
+// the cells from lo to hi along one axis; none or a negative number when the extent is negative (the ends saturate at the
+// range of int, so a span takes 33 bits)
+__device__ __forceinline__ int64_t bspan(float lo, float hi, float inv_cell) { return (int64_t)bcell(hi, inv_cell) - bcell(lo, inv_cell) + 1; }
 __device__ __forceinline__ uint32_t bhash(int32_t x, int32_t y, int32_t z) {
     return (uint32_t)x * 73856093u ^ (uint32_t)y * 19349663u ^ (uint32_t)z * 83492791u;
 }
@@ -580,11 +583,20 @@ __global__ void __launch_bounds__(T, CL == 1 && T <= 256 ? 2 : 1) k_box_step(BxA
         A.rot[b0 + i] = r;
         A.alo[b0 + i] = f4(lo, __uint_as_float((b.awake ? 1u : 0u) | (b.inv_m == 0.0f ? 2u : 0u))); A.ahi[b0 + i] = f4(hi, 0.0f);
         A.cand_n[b0 + i] = 0;
-        const uint64_t ne = (uint64_t)(bcell(hi.x, inv_cell) - bcell(lo.x, inv_cell) + 1) *
-                            (uint64_t)(bcell(hi.y, inv_cell) - bcell(lo.y, inv_cell) + 1) *
-                            (uint64_t)(bcell(hi.z, inv_cell) - bcell(lo.z, inv_cell) + 1);
-        if (ne > (uint64_t)BX_EPB * n) atomicOr(&Gp[G_ERR], (uint32_t)BXE_ENTRIES);
-        A.ecnt[b0 + i] = ne > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)ne;
+        // the grid entries the box counts for, saturated past the scene's; it has them only where all its spans are positive
+        const int64_t sp[3] = {bspan(lo.x, hi.x, inv_cell), bspan(lo.y, hi.y, inv_cell), bspan(lo.z, hi.z, inv_cell)};
+        const uint64_t most = (uint64_t)BX_EPB * n;
+        uint64_t ne = 1;
+        bool negative = false, any = true;
+        for (int k = 0; k < 3; k++) {
+            negative ^= sp[k] < 0; any &= sp[k] > 0;
+            ne *= (uint64_t)(sp[k] < 0 ? -sp[k] : sp[k]);
+            if (ne > most) ne = most + 1;
+        }
+        if (sp[0] == 0 || sp[1] == 0 || sp[2] == 0) ne = 0;
+        else if (negative) ne = most + 1;
+        if (ne > most) atomicOr(&Gp[G_ERR], (uint32_t)BXE_ENTRIES);
+        A.ecnt[b0 + i] = any ? (uint32_t)ne : 0u;
         atomicAdd((unsigned long long *)(Gp + G_NE), (unsigned long long)ne);
         A.wake[b0 + i] = 0;
         A.uf[b0 + i] = i;
@@ -625,13 +637,23 @@ __global__ void __launch_bounds__(T, CL == 1 && T <= 256 ? 2 : 1) k_box_step(BxA
     // ---- grid: one entry per body and covered cell, chained per hash slot
     for (uint32_t i = t; i < n; i += TT) {
         const P3 lo = xyz(A.alo[b0 + i]), hi = xyz(A.ahi[b0 + i]);
-        uint32_t e = atomicAdd(&Gp[G_TOT + 2], A.ecnt[b0 + i]);
+        const uint32_t ne = A.ecnt[b0 + i];
+        if (!ne) continue;
+        uint32_t e = atomicAdd(&Gp[G_TOT + 2], ne);
         const int32_t x0 = bcell(lo.x, inv_cell), y0 = bcell(lo.y, inv_cell), z0 = bcell(lo.z, inv_cell);
         const int32_t x1 = bcell(hi.x, inv_cell), y1 = bcell(hi.y, inv_cell), z1 = bcell(hi.z, inv_cell);
-        for (int32_t x = x0; x <= x1; x++) for (int32_t y = y0; y <= y1; y++) for (int32_t z = z0; z <= z1; z++) {
-            A.ent_body[e0 + e] = i;
-            A.ent_node[e0 + e] = make_int4(x, y, z, (int)atomicExch(&A.head[t0 + (bhash(x, y, z) & mask)], e));
-            e++;
+        // (a last cell may be the largest int, so the loops end at it and not past it)
+        for (int32_t x = x0;; x++) {
+            for (int32_t y = y0;; y++) {
+                for (int32_t z = z0;; z++) {
+                    A.ent_body[e0 + e] = i;
+                    A.ent_node[e0 + e] = make_int4(x, y, z, (int)atomicExch(&A.head[t0 + (bhash(x, y, z) & mask)], e));
+                    e++;
+                    if (z == z1) break;
+                }
+                if (y == y1) break;
+            }
+            if (x == x1) break;
         }
     }
     team_sync<CL>();
@@ -640,7 +662,8 @@ __global__ void __launch_bounds__(T, CL == 1 && T <= 256 ? 2 : 1) k_box_step(BxA
     // body's partners as they come, the counts are scanned, then the lists are written in order; a list of more than BX_SHORT
     // pairs (a static slab under a pile) is sorted by the team, and one that does not fit its row is walked for again.
     uint32_t *keep = (uint32_t *)(A.geom + (size_t)c0 * 20);
-    walk_pairs(A, b0, e0, ne_tot, inv_cell, t, TT, [&](uint32_t a, uint32_t b) {
+    const uint32_t n_ent = GV[G_TOT + 2];            // (a box that counts for entries without having any makes it less than ne_tot)
+    walk_pairs(A, b0, e0, n_ent, inv_cell, t, TT, [&](uint32_t a, uint32_t b) {
         const uint32_t k = atomicAdd(&A.cand_n[b0 + a], 1u);
         if (k < BX_KEEP) keep[(size_t)a * BX_KEEP + k] = b;
     });
@@ -681,7 +704,7 @@ __global__ void __launch_bounds__(T, CL == 1 && T <= 256 ? 2 : 1) k_box_step(BxA
     if (GV[G_TOT + 6]) {
         for (uint32_t a = t; a < n; a += TT) A.deg[s0 + a] = 0;
         team_sync<CL>();
-        walk_pairs(A, b0, e0, ne_tot, inv_cell, t, TT, [&](uint32_t a, uint32_t b) {
+        walk_pairs(A, b0, e0, n_ent, inv_cell, t, TT, [&](uint32_t a, uint32_t b) {
             const uint32_t off = A.cand_n[b0 + a];
             if (pairs_of(a, off) > BX_KEEP) A.cand_b[c0 + off + atomicAdd(&A.deg[s0 + a], 1u)] = b;
         });
