@@ -314,6 +314,8 @@ struct Work {
     DBuf<uint32_t> scan_a, scan_b, hist;
     uint64_t launches = 0;   // kernels launched by the scans and sorts
 };
+// room for scans of up to n_scan values and sorts of up to n_sort pairs, so that none of them allocates later
+cudaError_t work_reserve(Work &wk, size_t n_scan, size_t n_sort);
 // exclusive scan of n uint32 values (in place allowed); the total is written to *d_total if non-null
 cudaError_t exclusive_scan_u32(const uint32_t *in, uint32_t *out, size_t n, uint32_t *d_total, Work &wk, cudaStream_t s);
 // stable LSD radix sort of (key, value) pairs on key bits [0, bits). With in_alt null the result ends in keys/vals

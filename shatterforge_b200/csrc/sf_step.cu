@@ -43,8 +43,7 @@ struct StepState {
     DBuf<uint32_t> bsig;            // per (active scene, bucket) a 16-bit signature
     DBuf<float4> srec;
     DBuf<uint2> sent;
-    DBuf<uint4> slot_id;
-    DBuf<float4> slot_p, slot_n;
+    DBuf<float4> slots;             // a brick's first CSLOTS contacts: three words each, word by word
     // contacts, list order
     DBuf<uint32_t> ccount, coff;
     DBuf<uint32_t> L_a, L_b, L_bo, L_ba, L_bb;
@@ -55,8 +54,12 @@ struct StepState {
     DBuf<uint32_t> mflag, mpos, pair_start, cflag, cpos;
     DBuf<uint32_t> man_a, man_b, man_start, man_count, man_prio, man_color, man_round;
     DBuf<float4> S_n, S_t1, S_t2, S_ra, S_rb, S_j;
-    DBuf<uint4> M_id;               // per manifold in colour-list order: its bodies and contact count,
-    DBuf<float4> M_k;               // and its bodies' inverse masses and inertias, five float4 columns
+    // per manifold in colour-list order six columns: its bodies and contact count, and its bodies' inverse masses and
+    // inertias. In the room of the slots, which nothing reads once the contacts are placed, unless the contact capacity
+    // (a manifold has a contact at least) is more than they hold
+    DBuf<float4> man_rec;
+    float4 *man_records() { return man_rec.p ? man_rec.p : slots.p; }
+    size_t man_capacity() const { return (man_rec.p ? man_rec.n : slots.n) / 6; }
     DBuf<float4> vw;                // per active-list body: velocity and spin as the solve moves them (b_v, b_w keep those
                                     // before it)
     // contact reduction: per pair a big flag and its place among the big pairs, per big pair 27 best scores and 27
@@ -2427,6 +2430,7 @@ static cudaError_t grow_contacts(StepState *S, uint64_t need) {
     if (need <= S->capacity) return cudaSuccess;
     uint64_t cap = std::max<uint64_t>(need + need / 2, 4096);
     cudaError_t e;
+    S->capacity = 0;   // (after a growth that failed on the way, the next step with contacts grows again)
 #define G(buf) if ((e = S->buf.alloc(cap)) != cudaSuccess) return e
     G(L_a); G(L_b); G(L_bo); G(L_ba); G(L_bb); G(L_p); G(L_n);
     G(mkey); G(mkey_alt); G(perm); G(perm_alt); G(invperm); G(mflag); G(mpos); G(pair_start); G(cflag); G(cpos);
@@ -2437,6 +2441,7 @@ static cudaError_t grow_contacts(StepState *S, uint64_t need) {
 #undef G
     if ((e = S->red_slots.alloc(2 * 27 * (cap / 33 + 1))) != cudaSuccess) return e;
     if ((e = S->bm_list.alloc(2 * cap)) != cudaSuccess) return e;
+    if (cap > S->slots.n / 6 && (e = S->man_rec.alloc(6 * cap)) != cudaSuccess) return e;
     S->capacity = cap;
     return cudaSuccess;
 }
@@ -2463,7 +2468,7 @@ sf_status step_create(sf_world *w) {
     SF_CUDA(cudaFuncSetAttribute(k_small_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_SMEM));
     SF_CUDA(cudaFuncSetAttribute(k_contacts_gen_tab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEN_TAB_SMEM));
     SF_CUDA(S->srec.alloc(nd)); SF_CUDA(S->sent.alloc(nd));
-    SF_CUDA(S->slot_id.alloc((size_t)nd * CSLOTS)); SF_CUDA(S->slot_p.alloc((size_t)nd * CSLOTS)); SF_CUDA(S->slot_n.alloc((size_t)nd * CSLOTS));
+    SF_CUDA(S->slots.alloc((size_t)nd * CSLOTS * 3));
     SF_CUDA(S->ccount.alloc((size_t)nd + 1)); SF_CUDA(S->coff.alloc((size_t)nd + 1));
     SF_CUDA(S->bm_count.alloc((size_t)nb + 1)); SF_CUDA(S->bm_start.alloc((size_t)nb + 1)); SF_CUDA(S->bm_fill.alloc((size_t)nb + 1));
     const uint32_t mw = (w->P.max_colors + 31) / 32;
@@ -2497,7 +2502,6 @@ sf_status step_create(sf_world *w) {
     if (nb) SF_CUDA(cudaMemcpyAsync(S->body_off_of_body.p, off.data(), nb * 4, cudaMemcpyHostToDevice, s));
     uint64_t initial = w->P.contact_capacity ? w->P.contact_capacity : (uint64_t)std::max<uint32_t>(nd, 1) * 4;
     SF_CUDA(grow_contacts(S, initial));
-    SF_CUDA(S->M_id.alloc(std::min<uint64_t>(S->capacity, nd))); SF_CUDA(S->M_k.alloc(5 * S->M_id.n));
     int occ = 0;
     {
         auto *one = k_solve_team<1, SOLVE_TEAM_T1>;
@@ -2528,6 +2532,11 @@ sf_status step_create(sf_world *w) {
         int c[4], n = 0;
         for (int v = 1; v <= 4; v++) if (v <= top) c[n++] = v;
         S->solve_t.init(c, n);
+    }
+    if (w->P.contact_capacity) {
+        // a step with a fixed contact capacity allocates nothing
+        SF_CUDA(work_reserve(S->wk, std::max<size_t>({S->capacity, nd, (size_t)nsc * HSIZE, S->col_count.n}), S->capacity));
+        SF_CUDA(S->blk_dom.alloc((size_t)w->sms * std::min(S->solve_occ, S->jp_occ))); SF_CUDA(S->dom_of_act.alloc(nsc));
     }
     SF_CUDA(cudaStreamSynchronize(s));   // the host vector `off` is the copy's source
     return SF_OK;
@@ -2728,7 +2737,7 @@ static sf_status substep(sf_world *w, float h) {
     C.v = w->b_v.p; C.w = w->b_w.p; C.rot = w->b_rot.p; C.rad = w->b_rad.p; C.bstart = S->bstart.p; C.sig = S->bsig.p; C.srec = S->srec.p;
     C.sent = S->sent.p; C.ccount = S->ccount.p; C.coff = S->coff.p; C.wake = w->b_wake.p;
     C.sup = w->k_sup.p; C.frame = w->frame;
-    C.slot_id = S->slot_id.p; C.slot_p = S->slot_p.p; C.slot_n = S->slot_n.p;
+    C.slot_id = (uint4 *)S->slots.p; C.slot_p = S->slots.p + S->slots.n / 3; C.slot_n = C.slot_p + S->slots.n / 3;
     C.L_a = S->L_a.p; C.L_b = S->L_b.p; C.L_bo = S->L_bo.p; C.L_ba = S->L_ba.p; C.L_bb = S->L_bb.p; C.L_p = S->L_p.p; C.L_n = S->L_n.p;
     cudaEvent_t g0 = nullptr, g1 = nullptr;
     if (S->profile && n_awk) {
@@ -2925,11 +2934,6 @@ static sf_status substep(sf_world *w, float h) {
         prof_mark(w);
     }
     if (nc) {
-        // the solve's records are sized by the manifolds that occur (at most a contact each), not by the contact capacity
-        if (S->M_id.n < ncm) {
-            const size_t want = std::min<size_t>(S->capacity, 2 * (size_t)ncm + 65536);
-            SF_CUDA(S->M_id.alloc(want)); SF_CUDA(S->M_k.alloc(5 * want));
-        }
         PrepArgs PA;
         PA.nc = nc; PA.h = h; PA.nseg = nseg; PA.nm_p = S->dev.p + DV_MANIFOLDS; PA.perm = S->perm.p;
         PA.man_a = S->man_a.p; PA.man_b = S->man_b.p; PA.man_ca = S->man_ca.p; PA.man_cb = S->man_cb.p; PA.man_count = S->man_count.p; PA.L_p = S->L_p.p; PA.L_n = S->L_n.p;
@@ -2937,7 +2941,7 @@ static sf_status substep(sf_world *w, float h) {
         PA.jds_off = S->jds_off.p;
         PA.pos = w->b_pos.p; PA.v = w->b_v.p; PA.w = w->b_w.p; PA.im = w->b_im.p; PA.iiw = w->b_iiw.p;
         PA.S_n = S->S_n.p; PA.S_t1 = S->S_t1.p; PA.S_t2 = S->S_t2.p; PA.S_ra = S->S_ra.p; PA.S_rb = S->S_rb.p; PA.S_j = S->S_j.p;
-        PA.M_id = S->M_id.p; PA.M_k = S->M_k.p; PA.m_cap = S->M_id.n;
+        PA.M_id = (uint4 *)S->man_records(); PA.m_cap = S->man_capacity(); PA.M_k = S->man_records() + PA.m_cap;
         PA.invperm = S->invperm.p;
         const bool warm_read = w->P.warm_start && S->warm_valid;
         const StepState::WarmTable &WT = S->warm[S->warm_cur];
@@ -2965,7 +2969,7 @@ static sf_status substep(sf_world *w, float h) {
         SolveArgs A;
         A.iterations = w->P.iterations; A.dev = S->dev.p; A.col_start = S->col_start.p;
         A.blk_dom = S->blk_dom.p; A.dom_ncol = S->dom_ncol.p; A.cstride = cstride;
-        A.jds_off = S->jds_off.p; A.M_id = S->M_id.p; A.M_k = S->M_k.p; A.m_cap = S->M_id.n;
+        A.jds_off = S->jds_off.p; A.M_id = (const uint4 *)S->man_records(); A.m_cap = S->man_capacity(); A.M_k = S->man_records() + A.m_cap;
         A.S_n = S->S_n.p; A.S_t1 = S->S_t1.p; A.S_t2 = S->S_t2.p; A.S_ra = S->S_ra.p; A.S_rb = S->S_rb.p; A.S_j = S->S_j.p;
         A.vw = S->vw.p; A.nb = nb; A.gb = S->dom_gb.p; A.err = w->err.p;
         A.warm = w->P.warm_start ? 1u : 0u;

@@ -125,14 +125,19 @@ static cudaError_t scan_rec(const uint32_t *in, uint32_t *out, size_t n, uint32_
     return cudaGetLastError();
 }
 
+// words of the partial sums of a scan of n values, all its levels
+static size_t scan_words(size_t n) {
+    size_t need = 16;
+    while (n > (size_t)SCAN_TILE) { n = (n + SCAN_TILE - 1) / SCAN_TILE; need += n; }
+    return need;
+}
+
 cudaError_t exclusive_scan_u32(const uint32_t *in, uint32_t *out, size_t n, uint32_t *d_total, Work &wk, cudaStream_t s) {
     if (n == 0) {
         if (d_total) return cudaMemsetAsync(d_total, 0, sizeof(uint32_t), s);
         return cudaSuccess;
     }
-    size_t need = 0, m = n;
-    while (m > (size_t)SCAN_TILE) { m = (m + SCAN_TILE - 1) / SCAN_TILE; need += m; }
-    cudaError_t e = wk.scan_a.grow(need + 16);
+    cudaError_t e = wk.scan_a.grow(scan_words(n));
     if (e != cudaSuccess) return e;
     for (size_t q = n; ; q = (q + SCAN_TILE - 1) / SCAN_TILE) { wk.launches += q > (size_t)SCAN_TILE ? 2 : 1; if (q <= (size_t)SCAN_TILE) break; }
     return scan_rec(in, out, n, d_total, wk.scan_a.p, s);
@@ -210,13 +215,20 @@ __global__ void __launch_bounds__(RS_BLOCK) k_rs_scatter(const K *kin, const uin
     }
 }
 
+static size_t sort_words(size_t n) { return 256 * ((n + RS_TILE - 1) / RS_TILE); }
+
+cudaError_t work_reserve(Work &wk, size_t n_scan, size_t n_sort) {
+    const cudaError_t e = wk.hist.grow(sort_words(n_sort));
+    return e != cudaSuccess ? e : wk.scan_a.grow(scan_words(std::max(n_scan, sort_words(n_sort))));
+}
+
 template <class K>
 static cudaError_t radix_sort_impl(K *keys, uint32_t *vals, K *keys_alt, uint32_t *vals_alt, size_t n, int bits, Work &wk,
                                    cudaStream_t s, bool *in_alt) {
     if (in_alt) *in_alt = false;
     if (n <= 1 || bits <= 0) return cudaSuccess;
     unsigned nblocks = (unsigned)((n + RS_TILE - 1) / RS_TILE);
-    cudaError_t e = wk.hist.grow((size_t)256 * nblocks);
+    cudaError_t e = wk.hist.grow(sort_words(n));
     if (e != cudaSuccess) return e;
     int passes = (bits + 7) / 8;
     K *ki = keys, *ko = keys_alt;
