@@ -38,10 +38,13 @@ struct SorParams { double omega, tol; uint32_t max_sweeps, use_cap; };
 constexpr int SOR_CL = 8;                        // blocks of a structure's cluster, or SOR_CL_WIDE for large ones
 constexpr int SOR_CL_WIDE = 16;                  // a non-portable cluster size: structures of SOR_CL_WIDE_MIN bricks
 constexpr uint32_t SOR_CL_WIDE_MIN = 20000;
-constexpr int SOR_FORMS = 6;
-constexpr int SOR_FORM_T[SOR_FORMS] = {224, 480, 480, 608, 480, 480};
-constexpr int SOR_FORM_C[SOR_FORMS] = {1, 1, 2, 2, 3, 5};
-constexpr uint32_t SOR_CL_CAP = 2400;            // cells of one parity a block takes at most (the last form's T x C)
+constexpr int SOR_FORMS = 7;
+// The last two spill a part of what a cell keeps, and take more threads to hide it: with 16 blocks, us a sweep, a solid of 40^3
+// bricks (2,000 cells of one parity a block) 5.3 in 992 x 3 (480 x 5: 4.7, 736 x 4: 5.5), 125 x 4 x 125 (1,954) 4.1 (4.7, 4.6),
+// a trellis of 65,000 (3,144) 5.7 in 992 x 4 (480 x 9: 7.5, 736 x 6: 7.0, 992 x 5: 6.4).
+constexpr int SOR_FORM_T[SOR_FORMS] = {224, 480, 480, 608, 480, 992, 992};
+constexpr int SOR_FORM_C[SOR_FORMS] = {1, 1, 2, 2, 3, 3, 4};
+constexpr uint32_t SOR_CL_CAP = 3968;            // cells of one parity a block takes at most (the last form's T x C)
 constexpr int SOR_NCLS = 2 * SOR_FORMS;          // launch classes: a form, with 16 or 8 blocks
 
 // Per block of a structure's cluster: its cells and halo in the tables. Potentials in shared memory: [0] is 0 (the
@@ -1164,15 +1167,21 @@ static SorKernel sor_cluster_kernel(int form) {
         case 2: return k_sor_cluster<SOR_FORM_T[2], SOR_FORM_C[2]>;
         case 3: return k_sor_cluster<SOR_FORM_T[3], SOR_FORM_C[3]>;
         case 4: return k_sor_cluster<SOR_FORM_T[4], SOR_FORM_C[4]>;
-        default: return k_sor_cluster<SOR_FORM_T[5], SOR_FORM_C[5]>;
+        case 5: return k_sor_cluster<SOR_FORM_T[5], SOR_FORM_C[5]>;
+        default: return k_sor_cluster<SOR_FORM_T[6], SOR_FORM_C[6]>;
     }
 }
 static size_t sor_cluster_smem(uint32_t stride, uint32_t push, uint32_t ps) { return (size_t)stride * 16 + (size_t)push * 8 + (size_t)ps * 4; }
 constexpr size_t SOR_CL_SMEM = 200 * 1024;
 
 // The cluster path's tables, built on its first use: each structure's bricks in (y, z, x) order, which cuts a frame
-// along few links (a row of a slab, a storey's columns), split into ranges of equal size, one per block. A structure
-// with a block that fits no form of the kernel takes the grid kernel.
+// along few links (a row of a slab, a storey's columns), split into ranges of equal size, one per block. In a solid or thick
+// structure a layer is larger than a block's range, which then has all of the layers above and below as its halo: 60 x 12 x
+// 60 bricks have 8,221 potentials a block. Where a block does not fit that way, or where blocks of a 16-block cluster push
+// more than half of their cells, the bricks come in the order of the lattice's 8^3 chunks, whose ranges are compact (there
+// 3,978). Sweeps in the two orders, us: solids of 28^3 bricks 2.5, 1.7; 32^3 3.6, 2.1; 36^3 5.0, 3.9; 40^3 7.8, 5.3; 60 x 6 x
+// 60 3.6, 1.5; but frames, which push a tenth of their cells in either: 17,856 1.53, 1.75; 45,540 2.0, 3.0; and on 8
+// blocks 20^3 1.41, 1.46. A structure with a block that fits no form of the kernel in either order takes the grid kernel.
 static sf_status sor_cluster_tables(sf_world *w) {
     SorState *st = w->sor;
     for (int f = 0; f < SOR_FORMS; f++) {
@@ -1207,10 +1216,10 @@ static sf_status sor_cluster_tables(sf_world *w) {
         for (uint32_t i = 0; i < w->scenes[q].n_static; i++) scene_of[w->scenes[q].static_off + i] = q;
     std::vector<std::vector<uint32_t>> bricks(nst);
     for (uint32_t i = 0; i < ns; i++) if (w->h_sid[i] >= 0) bricks[w->h_sid[i]].push_back(i);
-    auto key = [&](uint32_t i) {
+    auto key = [&](uint32_t i, bool chunks) {
         int x, y, z;
         unpack_cell(w->h_s_cell[i], x, y, z);
-        return ((uint64_t)y << 20) | ((uint64_t)z << 10) | (uint64_t)x;
+        return chunks ? (uint64_t)chunk_slot(x, y, z) * 512 + cell_in_chunk(x, y, z) : ((uint64_t)y << 20) | ((uint64_t)z << 10) | (uint64_t)x;
     };
     auto cpos_of = [&](uint32_t sc, int x, int y, int z) -> uint32_t {   // chunk * 512 + cell, or NONE
         if (!inb(x, y, z)) return NONE;
@@ -1226,14 +1235,16 @@ static sf_status sor_cluster_tables(sf_world *w) {
     st->h_guess.assign(nst, 0.0);
     st->h_last_sweeps.assign(nst, 0);
     const int D[6][3] = {{1, 0, 0}, {-1, 0, 0}, {0, 1, 0}, {0, -1, 0}, {0, 0, 1}, {0, 0, -1}};
-    for (uint32_t q = 0; q < nst; q++) {
+    enum { LAYERS_IF_THIN, CHUNKS, LAYERS };
+    auto lay_out = [&](uint32_t q, int order) -> bool {   // false: a block does not fit in this order
+        const bool chunks = order == CHUNKS;
         // links join bricks of one structure only (a bond needs equal structure ids), so every link of a listed
         // cell ends at a listed cell
         std::vector<uint32_t> &b = bricks[q];
         const uint32_t n = (uint32_t)b.size();
-        if (n == 0 || n >= 65535u) continue;
+        if (n == 0 || n >= 65535u) return true;
         keys.clear();
-        for (uint32_t i : b) keys.push_back(key(i) << 24 | (uint32_t)(keys.size()));
+        for (uint32_t i : b) keys.push_back(key(i, chunks) << 24 | (uint32_t)(keys.size()));
         std::sort(keys.begin(), keys.end());
         {
             std::vector<uint32_t> o(b);
@@ -1351,9 +1362,10 @@ static sf_status sor_cluster_tables(sf_world *w) {
             ci.push = std::max(ci.push, B.npush);
             ci.ps = std::max(ci.ps, B.push_even + B.push_odd + 1);
         }
+        if (order == LAYERS_IF_THIN && ncl == (uint32_t)SOR_CL_WIDE && 2 * ci.push > pr) fits = false;
         if (!fits || sor_cluster_smem(ci.stride, ci.push, ci.ps) > SOR_CL_SMEM) {
             cpos.resize(c_at); hpos.resize(h_at); hface.resize(h_at); ps.resize(ps_at); push.resize(p_at); nbr.resize(n_at);
-            continue;
+            return false;
         }
         int form = 0;
         while (ci.half > (uint32_t)(SOR_FORM_T[form] * SOR_FORM_C[form])) form++;
@@ -1363,7 +1375,10 @@ static sf_status sor_cluster_tables(sf_world *w) {
         // to 1e-6 with omega 1.7 the 37 buildings of the lattice take 5 to 9 sweeps per height times the root of their
         // bricks per footing
         st->h_guess[q] = 7.0 * (yhi - ylo + 1) * std::sqrt((double)n / std::max(foot, 1u));
-    }
+        return true;
+    };
+    for (uint32_t q = 0; q < nst; q++)
+        if (!lay_out(q, LAYERS_IF_THIN) && !lay_out(q, CHUNKS)) lay_out(q, LAYERS);
     cudaStream_t s = w->stream;
     auto up = [&](auto &d, const auto &h) -> cudaError_t {
         cudaError_t e = d.alloc(std::max<size_t>(h.size(), 1));
