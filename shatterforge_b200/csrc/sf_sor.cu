@@ -1174,7 +1174,27 @@ static SorKernel sor_cluster_kernel(int form) {
 static size_t sor_cluster_smem(uint32_t stride, uint32_t push, uint32_t ps) { return (size_t)stride * 16 + (size_t)push * 8 + (size_t)ps * 4; }
 constexpr size_t SOR_CL_SMEM = 200 * 1024;
 
-// The cluster path's tables, built on its first use: each structure's bricks in (y, z, x) order, which cuts a frame
+// The cluster path's tables on the host, of all structures: the cells of each block and its halo (see SorBlock), and what a
+// launch needs to know of a structure.
+struct SorTables {
+    std::vector<uint32_t> cpos, hpos, ps, push;
+    std::vector<uint16_t> nbr;
+    std::vector<uint8_t> hface;
+    std::vector<SorBlock> blk;
+    std::vector<SorState::ClInfo> info;
+    std::vector<double> guess;
+};
+// the static bricks as the tables need them
+struct SorBricks {
+    uint32_t ns, nst;
+    const uint32_t *cell, *scene;                // packed lattice cells, scenes
+    const int32_t *sid;
+    const uint8_t *mat;
+    const uint32_t *ctab;                        // NCT words a scene: chunk + 1
+    bool wide_ok;
+};
+
+// Each structure's bricks come in (y, z, x) order, which cuts a frame
 // along few links (a row of a slab, a storey's columns), split into ranges of equal size, one per block. In a solid or thick
 // structure a layer is larger than a block's range, which then has all of the layers above and below as its halo: 60 x 12 x
 // 60 bricks have 8,221 potentials a block. Where a block does not fit that way, or where blocks of a 16-block cluster push
@@ -1182,6 +1202,209 @@ constexpr size_t SOR_CL_SMEM = 200 * 1024;
 // 3,978). Sweeps in the two orders, us: solids of 28^3 bricks 2.5, 1.7; 32^3 3.6, 2.1; 36^3 5.0, 3.9; 40^3 7.8, 5.3; 60 x 6 x
 // 60 3.6, 1.5; but frames, which push a tenth of their cells in either: 17,856 1.53, 1.75; 45,540 2.0, 3.0; and on 8
 // blocks 20^3 1.41, 1.46. A structure with a block that fits no form of the kernel in either order takes the grid kernel.
+// The first solve of a world pays for these tables, so they are counted first and written in place, with neighbours found
+// along the sorted bricks: 37 buildings of 378,000 bricks in 24 ms on one core, against 60 with searches a neighbour and
+// growing vectors.
+static void sor_build_tables(const SorBricks &W, SorTables &T) {
+    const uint32_t nst = W.nst;
+    T.blk.assign(std::max<size_t>((size_t)nst * SOR_CL_WIDE, 1), SorBlock{});
+    T.info.assign(nst, SorState::ClInfo{});
+    T.guess.assign(nst, 0.0);
+    // the bricks by structure, ascending (and so scene by scene)
+    std::vector<uint32_t> first((size_t)nst + 1, 0), brick;
+    for (uint32_t i = 0; i < W.ns; i++) if (W.sid[i] >= 0) first[W.sid[i] + 1]++;
+    for (uint32_t q = 0; q < nst; q++) first[q + 1] += first[q];
+    const uint32_t total = first[nst];
+    brick.resize(total);
+    {
+        std::vector<uint32_t> at(first.begin(), first.end() - 1);
+        for (uint32_t i = 0; i < W.ns; i++) if (W.sid[i] >= 0) brick[at[W.sid[i]]++] = i;
+    }
+    T.cpos.resize(total);
+    T.nbr.resize((size_t)total * 6);
+    size_t c_at = 0;
+    constexpr uint32_t NO = 0xFFFFu;
+    auto key_of = [&](uint32_t i) -> uint64_t {
+        const uint32_t c = W.cell[i];
+        return ((uint64_t)W.scene[i] << 32) | ((c >> 10) & 255u) << 20 | (c >> 18) << 10 | (c & 1023u);
+    };
+    // of the k-th brick of a structure in (scene, y, z, x) order
+    std::vector<uint64_t> key, order_key;
+    std::vector<uint32_t> tmp, cp, ord, list, toff, count;
+    std::vector<uint16_t> face, place, tplace;
+    std::vector<uint8_t> rank, odd, slug, trank, tface;
+    for (uint32_t q = 0; q < nst; q++) {
+        // links join bricks of one structure only (a bond needs equal structure ids), so every link of a listed
+        // cell ends at a listed cell
+        const uint32_t n = first[q + 1] - first[q];
+        if (n == 0 || n >= 65535u) continue;
+        uint32_t *b = brick.data() + first[q];
+        key.resize(n);
+        bool sorted = true;
+        for (uint32_t k = 0; k < n; k++) { key[k] = key_of(b[k]); sorted &= k == 0 || key[k - 1] < key[k]; }
+        if (!sorted) {
+            tmp.resize(n);
+            for (int shift : {0, 10, 20}) {       // by x, z, y, each pass stable
+                count.assign(1025, 0);
+                for (uint32_t k = 0; k < n; k++) count[((key[k] >> shift) & 1023u) + 1]++;
+                for (uint32_t c = 0; c < 1024; c++) count[c + 1] += count[c];
+                for (uint32_t k = 0; k < n; k++) tmp[count[(key[k] >> shift) & 1023u]++] = b[k];
+                std::copy(tmp.begin(), tmp.end(), b);
+                for (uint32_t k = 0; k < n; k++) key[k] = key_of(b[k]);
+            }
+            if (W.scene[*std::min_element(b, b + n)] != W.scene[*std::max_element(b, b + n)]) {
+                std::stable_sort(b, b + n, [&](uint32_t u, uint32_t v) { return W.scene[u] < W.scene[v]; });
+                for (uint32_t k = 0; k < n; k++) key[k] = key_of(b[k]);
+            }
+        }
+        cp.resize(n); odd.resize(n); slug.resize(n);
+        int ylo = NY, yhi = -1;
+        uint32_t foot = 0;
+        for (uint32_t k = 0; k < n; k++) {
+            int x, y, z;
+            unpack_cell(W.cell[b[k]], x, y, z);
+            cp[k] = (W.ctab[(size_t)W.scene[b[k]] * NCT + chunk_slot(x, y, z)] - 1) * 512 + cell_in_chunk(x, y, z);
+            odd[k] = (uint8_t)((x + y + z) & 1);
+            slug[k] = W.mat[b[k]] >= SLUG;
+            ylo = std::min(ylo, y); yhi = std::max(yhi, y);
+            foot += y == 0 ? 1 : 0;
+        }
+        // the bricks at the faces +x, -x, +y, -y, +z, -z: the keys ascend, so do those one step along an axis
+        face.assign((size_t)n * 6, (uint16_t)NO);
+        for (int axis = 0; axis < 3; axis++) {
+            const uint64_t step = axis == 0 ? 1u : axis == 1 ? 1u << 20 : 1u << 10;
+            for (uint32_t k = 0, j = 0; k < n; k++) {
+                while (j < n && key[j] < key[k] + step) j++;
+                if (j == n) break;
+                if (key[j] == key[k] + step) { face[(size_t)k * 6 + 2 * axis] = (uint16_t)j; face[(size_t)j * 6 + 2 * axis + 1] = (uint16_t)k; }
+            }
+        }
+        const uint32_t ncl = (W.wide_ok && n >= SOR_CL_WIDE_MIN) ? (uint32_t)SOR_CL_WIDE : (uint32_t)SOR_CL;
+        const uint32_t pr = (n + ncl - 1) / ncl;
+        ord.resize(n); rank.resize(n); toff.resize((size_t)n + 1); place.resize(n); list.resize(n);
+        for (uint32_t k = 0; k < n; k++) ord[k] = k;
+        // per block: cells by parity, pushed and not; pushes; halo by parity of its cells
+        struct Counts { uint32_t cell[4], push, halo[2]; } N[SOR_CL_WIDE];
+        SorState::ClInfo ci;
+        bool fits = false;
+        enum { LAYERS_IF_THIN, CHUNKS, LAYERS };
+        for (int order = LAYERS_IF_THIN; order <= LAYERS && !fits; order++) {
+            if (order == LAYERS) for (uint32_t k = 0; k < n; k++) ord[k] = k;
+            if (order == CHUNKS) {
+                order_key.resize(n);
+                for (uint32_t k = 0; k < n; k++) {
+                    int x, y, z;
+                    unpack_cell(W.cell[b[k]], x, y, z);
+                    order_key[k] = ((key[k] >> 32) << 42) | ((uint64_t)chunk_slot(x, y, z) << 25) | ((uint64_t)cell_in_chunk(x, y, z) << 16) | k;
+                }
+                std::sort(order_key.begin(), order_key.end());
+                for (uint32_t k = 0; k < n; k++) ord[k] = (uint32_t)(order_key[k] & 0xFFFFu);
+            }
+            for (uint32_t p = 0; p < n; p++) rank[ord[p]] = (uint8_t)(p / pr);
+            // the blocks a brick's value goes to, ascending, each with the faces behind which it lies with a brick that a
+            // solve may update (a brick of SLUG or above is read but never updated)
+            std::memset(N, 0, sizeof N);
+            trank.clear(); tface.clear();
+            for (uint32_t k = 0; k < n; k++) {
+                const uint32_t own = rank[k], t0 = (uint32_t)trank.size();
+                toff[k] = t0;
+                for (int d = 0; d < 6; d++) {
+                    const uint32_t j = face[(size_t)k * 6 + d];
+                    if (j == NO || rank[j] == own) continue;
+                    const uint8_t r = rank[j], f = slug[j] ? 0 : (uint8_t)(1u << d);
+                    uint32_t t = t0;
+                    while (t < trank.size() && trank[t] < r) t++;
+                    if (t == trank.size() || trank[t] != r) { trank.insert(trank.begin() + t, r); tface.insert(tface.begin() + t, f); }
+                    else tface[t] |= f;
+                }
+                const uint32_t m = (uint32_t)trank.size() - t0;
+                N[own].cell[2 * odd[k] + (m ? 0 : 1)]++;
+                N[own].push += m;
+                for (uint32_t t = t0; t < t0 + m; t++) N[trank[t]].halo[odd[k]]++;
+            }
+            toff[n] = (uint32_t)trank.size();
+            ci = SorState::ClInfo{};
+            for (uint32_t r = 0; r < ncl; r++) {
+                const Counts &c = N[r];
+                const uint32_t even = c.cell[0] + c.cell[1], all = even + c.cell[2] + c.cell[3];
+                ci.half = std::max(ci.half, std::max(even, all - even));
+                ci.stride = std::max(ci.stride, 1 + all + c.halo[0] + c.halo[1]);
+                ci.push = std::max(ci.push, c.push);
+                ci.ps = std::max(ci.ps, c.cell[0] + c.cell[2] + 1);
+            }
+            // (a potential's byte offset takes 16 bits)
+            fits = ci.half <= SOR_CL_CAP && ci.stride <= 0x2000u && sor_cluster_smem(ci.stride, ci.push, ci.ps) <= SOR_CL_SMEM;
+            if (order == LAYERS_IF_THIN && ncl == (uint32_t)SOR_CL_WIDE && 2 * ci.push > pr) fits = false;
+        }
+        if (!fits) continue;
+        // places: a block's cells even then odd, each with the pushed cells first; its halo's, even first
+        uint32_t next[SOR_CL_WIDE][4], hnext[SOR_CL_WIDE][2], h0 = (uint32_t)T.hpos.size(), ps0 = (uint32_t)T.ps.size(), p0 = (uint32_t)T.push.size();
+        uint32_t c0 = (uint32_t)c_at;
+        for (uint32_t r = 0; r < ncl; r++) {
+            const Counts &c = N[r];
+            SorBlock &B = T.blk[(size_t)q * SOR_CL_WIDE + r];
+            B.cell0 = c0; B.neven = c.cell[0] + c.cell[1]; B.ncell = B.neven + c.cell[2] + c.cell[3];
+            B.push_even = c.cell[0]; B.push_odd = c.cell[2]; B.npush = c.push;
+            B.halo0 = h0; B.halo_even = c.halo[0]; B.nhalo = c.halo[0] + c.halo[1];
+            B.ps0 = ps0; B.push0 = p0;
+            uint32_t at = 0;
+            for (int k = 0; k < 4; k++) { next[r][k] = at; at += c.cell[k]; }
+            hnext[r][0] = 0; hnext[r][1] = c.halo[0];
+            c0 += B.ncell; h0 += B.nhalo; p0 += c.push; ps0 += c.cell[0] + c.cell[2] + 1;
+        }
+        T.hpos.resize(h0); T.hface.resize(h0); T.ps.resize(ps0); T.push.resize(p0);
+        for (uint32_t p = 0; p < n; p++) {
+            const uint32_t k = ord[p], r = rank[k];
+            const uint32_t at = next[r][2 * odd[k] + (toff[k + 1] > toff[k] ? 0 : 1)]++;
+            place[k] = (uint16_t)(1 + at);
+            list[r * pr + at] = k;
+        }
+        tplace.resize(trank.size());
+        for (uint32_t k = 0; k < n; k++)
+            for (uint32_t t = toff[k]; t < toff[k + 1]; t++) {
+                const SorBlock &B = T.blk[(size_t)q * SOR_CL_WIDE + trank[t]];
+                const uint32_t at = hnext[trank[t]][odd[k]]++;
+                tplace[t] = (uint16_t)(1 + B.ncell + at);
+                T.hpos[B.halo0 + at] = cp[k];
+                T.hface[B.halo0 + at] = tface[t];
+            }
+        for (uint32_t r = 0; r < ncl; r++) {
+            const SorBlock &B = T.blk[(size_t)q * SOR_CL_WIDE + r];
+            uint32_t c = B.ps0, e = B.push0;
+            for (uint32_t u = 0; u < B.ncell; u++) {
+                const uint32_t k = list[r * pr + u];
+                T.cpos[B.cell0 + u] = cp[k];
+                uint16_t *nb = T.nbr.data() + (size_t)(B.cell0 + u) * 6;
+                for (int d = 0; d < 6; d++) {
+                    const uint32_t j = face[(size_t)k * 6 + d];
+                    if (j == NO) { nb[d] = 0; continue; }
+                    if (rank[j] == r) { nb[d] = place[j]; continue; }
+                    uint32_t t = toff[j];
+                    while (trank[t] != r) t++;
+                    nb[d] = tplace[t];
+                }
+                if (toff[k + 1] == toff[k]) continue;
+                T.ps[c++] = e - B.push0;
+                for (uint32_t t = toff[k]; t < toff[k + 1]; t++)
+                    T.push[e++] = ((uint32_t)trank[t] << 24) | ((uint32_t)tface[t] << 16) | tplace[t];
+            }
+            T.ps[c] = e - B.push0;
+        }
+        c_at += n;
+        int form = 0;
+        while (ci.half > (uint32_t)(SOR_FORM_T[form] * SOR_FORM_C[form])) form++;
+        ci.n = n;
+        ci.cls = 2 * (uint32_t)form + (ncl == (uint32_t)SOR_CL_WIDE ? 1u : 0u);
+        T.info[q] = ci;
+        // to 1e-6 with omega 1.7 the 37 buildings of the lattice take 5 to 9 sweeps per height times the root of their
+        // bricks per footing
+        T.guess[q] = 7.0 * (yhi - ylo + 1) * std::sqrt((double)n / std::max(foot, 1u));
+    }
+    T.cpos.resize(c_at);
+    T.nbr.resize(c_at * 6);
+}
+
+// the tables on the device, built on the path's first use
 static sf_status sor_cluster_tables(sf_world *w) {
     SorState *st = w->sor;
     for (int f = 0; f < SOR_FORMS; f++) {
@@ -1205,188 +1428,26 @@ static sf_status sor_cluster_tables(sf_world *w) {
         st->wide_ok = nc > 0;
     }
     const uint32_t nst = w->n_struct, ns = w->ns;
-    std::vector<uint32_t> h_ctab((size_t)w->n_scenes * NCT), h_cpool((size_t)std::max<uint32_t>(w->n_chunks, 1) * 512);
+    std::vector<uint32_t> h_ctab((size_t)w->n_scenes * NCT), scene(ns);
+    std::vector<uint8_t> h_mat(std::max<uint32_t>(ns, 1));
     SF_CUDA(cudaStreamSynchronize(w->stream));
     SF_CUDA(cudaMemcpy(h_ctab.data(), w->ctab.p, h_ctab.size() * 4, cudaMemcpyDeviceToHost));
-    if (w->n_chunks) SF_CUDA(cudaMemcpy(h_cpool.data(), w->cpool.p, (size_t)w->n_chunks * 512 * 4, cudaMemcpyDeviceToHost));
-    std::vector<uint8_t> h_mat(std::max<uint32_t>(ns, 1));
     if (ns) SF_CUDA(cudaMemcpy(h_mat.data(), w->s_mat.p, ns, cudaMemcpyDeviceToHost));
-    std::vector<uint32_t> scene_of(ns, 0);
     for (uint32_t q = 0; q < w->n_scenes; q++)
-        for (uint32_t i = 0; i < w->scenes[q].n_static; i++) scene_of[w->scenes[q].static_off + i] = q;
-    std::vector<std::vector<uint32_t>> bricks(nst);
-    for (uint32_t i = 0; i < ns; i++) if (w->h_sid[i] >= 0) bricks[w->h_sid[i]].push_back(i);
-    auto key = [&](uint32_t i, bool chunks) {
-        int x, y, z;
-        unpack_cell(w->h_s_cell[i], x, y, z);
-        return chunks ? (uint64_t)chunk_slot(x, y, z) * 512 + cell_in_chunk(x, y, z) : ((uint64_t)y << 20) | ((uint64_t)z << 10) | (uint64_t)x;
-    };
-    auto cpos_of = [&](uint32_t sc, int x, int y, int z) -> uint32_t {   // chunk * 512 + cell, or NONE
-        if (!inb(x, y, z)) return NONE;
-        const uint32_t t = h_ctab[(size_t)sc * NCT + chunk_slot(x, y, z)];
-        return t ? (t - 1) * 512 + cell_in_chunk(x, y, z) : NONE;
-    };
-    std::vector<uint32_t> rank_of(ns, NONE), place(ns, 0), face_nbr((size_t)ns * 6, NONE), cpos, hpos, ps, push;
-    std::vector<uint64_t> keys;
-    std::vector<SorBlock> blk(std::max<size_t>((size_t)nst * SOR_CL_WIDE, 1), SorBlock{});
-    std::vector<uint16_t> nbr;
-    std::vector<uint8_t> hface;
-    st->h_cl.assign(nst, SorState::ClInfo{});
-    st->h_guess.assign(nst, 0.0);
+        std::fill_n(scene.begin() + w->scenes[q].static_off, w->scenes[q].n_static, q);
+    SorTables T;
+    sor_build_tables({ns, nst, w->h_s_cell.data(), scene.data(), w->h_sid.data(), h_mat.data(), h_ctab.data(), st->wide_ok}, T);
+    st->h_cl = std::move(T.info);
+    st->h_guess = std::move(T.guess);
     st->h_last_sweeps.assign(nst, 0);
-    const int D[6][3] = {{1, 0, 0}, {-1, 0, 0}, {0, 1, 0}, {0, -1, 0}, {0, 0, 1}, {0, 0, -1}};
-    enum { LAYERS_IF_THIN, CHUNKS, LAYERS };
-    auto lay_out = [&](uint32_t q, int order) -> bool {   // false: a block does not fit in this order
-        const bool chunks = order == CHUNKS;
-        // links join bricks of one structure only (a bond needs equal structure ids), so every link of a listed
-        // cell ends at a listed cell
-        std::vector<uint32_t> &b = bricks[q];
-        const uint32_t n = (uint32_t)b.size();
-        if (n == 0 || n >= 65535u) return true;
-        keys.clear();
-        for (uint32_t i : b) keys.push_back(key(i, chunks) << 24 | (uint32_t)(keys.size()));
-        std::sort(keys.begin(), keys.end());
-        {
-            std::vector<uint32_t> o(b);
-            for (uint32_t k = 0; k < n; k++) b[k] = o[keys[k] & 0xFFFFFFu];
-        }
-        const uint32_t ncl = (st->wide_ok && n >= SOR_CL_WIDE_MIN) ? (uint32_t)SOR_CL_WIDE : (uint32_t)SOR_CL;
-        const uint32_t pr = (n + ncl - 1) / ncl;
-        for (uint32_t k = 0; k < n; k++) rank_of[b[k]] = k / pr;
-        auto parity = [&](uint32_t i) {
-            int x, y, z;
-            unpack_cell(w->h_s_cell[i], x, y, z);
-            return (x + y + z) & 1;
-        };
-        for (uint32_t i : b) {   // the structure's bricks at the faces, or NONE
-            int x, y, z;
-            unpack_cell(w->h_s_cell[i], x, y, z);
-            for (int d = 0; d < 6; d++) {
-                const uint32_t c = cpos_of(scene_of[i], x + D[d][0], y + D[d][1], z + D[d][2]);
-                const uint32_t j1 = c == NONE ? 0u : h_cpool[c];
-                face_nbr[(size_t)i * 6 + d] = j1 && w->h_sid[j1 - 1] == (int32_t)q ? j1 - 1 : NONE;
-            }
-        }
-        auto nbr_of = [&](uint32_t i, int d) -> uint32_t { return face_nbr[(size_t)i * 6 + d]; };
-        // the faces of a brick behind which block r lies with a brick that a solve may update (a brick of SLUG or above is
-        // read but never updated)
-        auto faces = [&](uint32_t i, uint32_t r) -> uint32_t {
-            uint32_t m = 0;
-            for (int d = 0; d < 6; d++) {
-                const uint32_t j = nbr_of(i, d);
-                if (j != NONE && rank_of[j] == r && h_mat[j] < SLUG) m |= 1u << d;
-            }
-            return m;
-        };
-        // the blocks a brick's value goes to, in ascending order
-        auto targets = [&](uint32_t i, uint32_t *to) -> uint32_t {
-            uint32_t m = 0;
-            for (int d = 0; d < 6; d++) {
-                const uint32_t j = nbr_of(i, d);
-                if (j != NONE && rank_of[j] != rank_of[i]) to[m++] = rank_of[j];
-            }
-            if (m < 2) return m;
-            std::sort(to, to + m);
-            return (uint32_t)(std::unique(to, to + m) - to);
-        };
-        uint32_t to[6];
-        SorState::ClInfo ci;
-        const size_t c_at = cpos.size(), h_at = hpos.size(), ps_at = ps.size(), p_at = push.size(), n_at = nbr.size();
-        // order of each range: even then odd, each with the pushed cells first; then the blocks' halos, whose places
-        // follow the cells
-        for (uint32_t r = 0; r < ncl; r++) {
-            SorBlock &B = blk[(size_t)q * SOR_CL_WIDE + r];
-            auto lo = b.begin() + std::min(n, r * pr), hi = b.begin() + std::min(n, (r + 1) * pr);
-            std::vector<uint32_t> o[4];
-            for (auto it = lo; it != hi; ++it) o[2 * parity(*it) + (targets(*it, to) ? 0 : 1)].push_back(*it);
-            B = SorBlock{};
-            B.cell0 = (uint32_t)(c_at + (lo - b.begin()));
-            for (const std::vector<uint32_t> &part : o)
-                for (uint32_t i : part) { *(lo + B.ncell) = i; place[i] = 1 + B.ncell++; }
-            B.neven = (uint32_t)(o[0].size() + o[1].size());
-            B.push_even = (uint32_t)o[0].size();
-            B.push_odd = (uint32_t)o[2].size();
-            ci.half = std::max(ci.half, std::max(B.neven, B.ncell - B.neven));
-        }
-        std::vector<std::vector<uint32_t>> hplace(ncl);   // per block: the halo bricks, even first, ascending by brick
-        auto halo_before = [&](uint32_t u, uint32_t v) { return parity(u) != parity(v) ? parity(u) < parity(v) : u < v; };
-        for (uint32_t k = 0; k < n; k++) {
-            const uint32_t m = targets(b[k], to);
-            for (uint32_t t = 0; t < m; t++) hplace[to[t]].push_back(b[k]);
-        }
-        for (uint32_t r = 0; r < ncl; r++) {
-            SorBlock &B = blk[(size_t)q * SOR_CL_WIDE + r];
-            std::sort(hplace[r].begin(), hplace[r].end(), halo_before);
-            B.halo0 = (uint32_t)hpos.size();
-            B.nhalo = (uint32_t)hplace[r].size();
-            B.halo_even = 0;
-            for (uint32_t i : hplace[r]) {
-                if (!parity(i)) B.halo_even++;
-                int x, y, z;
-                unpack_cell(w->h_s_cell[i], x, y, z);
-                hpos.push_back(cpos_of(scene_of[i], x, y, z));
-                hface.push_back((uint8_t)faces(i, r));
-            }
-            ci.stride = std::max(ci.stride, 1 + B.ncell + B.nhalo);
-        }
-        auto place_in = [&](uint32_t i, uint32_t r) -> uint32_t {
-            if (rank_of[i] == r) return place[i];
-            const std::vector<uint32_t> &hp = hplace[r];
-            return 1 + blk[(size_t)q * SOR_CL_WIDE + r].ncell + (uint32_t)(std::lower_bound(hp.begin(), hp.end(), i, halo_before) - hp.begin());
-        };
-        bool fits = ci.half <= SOR_CL_CAP && ci.stride <= 0x2000u;   // (a potential's byte offset takes 16 bits)
-        int ylo = NY, yhi = -1;
-        uint32_t foot = 0;
-        for (uint32_t r = 0; r < ncl && fits; r++) {
-            SorBlock &B = blk[(size_t)q * SOR_CL_WIDE + r];
-            B.ps0 = (uint32_t)ps.size();
-            B.push0 = (uint32_t)push.size();
-            for (uint32_t k = 0; k < B.ncell; k++) {
-                const uint32_t i = b[B.cell0 - c_at + k];
-                int x, y, z;
-                unpack_cell(w->h_s_cell[i], x, y, z);
-                ylo = std::min(ylo, y); yhi = std::max(yhi, y);
-                foot += y == 0 ? 1 : 0;
-                cpos.push_back(cpos_of(scene_of[i], x, y, z));
-                for (int d = 0; d < 6; d++) {
-                    const uint32_t j = nbr_of(i, d);
-                    nbr.push_back(j == NONE ? (uint16_t)0 : (uint16_t)place_in(j, r));
-                }
-                const uint32_t m = targets(i, to);
-                if (!m) continue;
-                ps.push_back((uint32_t)push.size() - B.push0);
-                for (uint32_t t = 0; t < m; t++) push.push_back((to[t] << 24) | (faces(i, to[t]) << 16) | place_in(i, to[t]));
-            }
-            B.npush = (uint32_t)push.size() - B.push0;
-            ps.push_back(B.npush);
-            ci.push = std::max(ci.push, B.npush);
-            ci.ps = std::max(ci.ps, B.push_even + B.push_odd + 1);
-        }
-        if (order == LAYERS_IF_THIN && ncl == (uint32_t)SOR_CL_WIDE && 2 * ci.push > pr) fits = false;
-        if (!fits || sor_cluster_smem(ci.stride, ci.push, ci.ps) > SOR_CL_SMEM) {
-            cpos.resize(c_at); hpos.resize(h_at); hface.resize(h_at); ps.resize(ps_at); push.resize(p_at); nbr.resize(n_at);
-            return false;
-        }
-        int form = 0;
-        while (ci.half > (uint32_t)(SOR_FORM_T[form] * SOR_FORM_C[form])) form++;
-        ci.n = n;
-        ci.cls = 2 * (uint32_t)form + (ncl == (uint32_t)SOR_CL_WIDE ? 1u : 0u);
-        st->h_cl[q] = ci;
-        // to 1e-6 with omega 1.7 the 37 buildings of the lattice take 5 to 9 sweeps per height times the root of their
-        // bricks per footing
-        st->h_guess[q] = 7.0 * (yhi - ylo + 1) * std::sqrt((double)n / std::max(foot, 1u));
-        return true;
-    };
-    for (uint32_t q = 0; q < nst; q++)
-        if (!lay_out(q, LAYERS_IF_THIN) && !lay_out(q, CHUNKS)) lay_out(q, LAYERS);
     cudaStream_t s = w->stream;
     auto up = [&](auto &d, const auto &h) -> cudaError_t {
         cudaError_t e = d.alloc(std::max<size_t>(h.size(), 1));
         if (e == cudaSuccess && !h.empty()) e = cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice, s);
         return e;
     };
-    SF_CUDA(up(st->cl_cpos, cpos)); SF_CUDA(up(st->cl_hpos, hpos)); SF_CUDA(up(st->cl_ps, ps)); SF_CUDA(up(st->cl_push, push));
-    SF_CUDA(up(st->cl_blk, blk)); SF_CUDA(up(st->cl_nbr, nbr)); SF_CUDA(up(st->cl_hface, hface));
+    SF_CUDA(up(st->cl_cpos, T.cpos)); SF_CUDA(up(st->cl_hpos, T.hpos)); SF_CUDA(up(st->cl_ps, T.ps)); SF_CUDA(up(st->cl_push, T.push));
+    SF_CUDA(up(st->cl_blk, T.blk)); SF_CUDA(up(st->cl_nbr, T.nbr)); SF_CUDA(up(st->cl_hface, T.hface));
     SF_CUDA(st->cl_list.alloc(std::max<uint32_t>(nst, 1)));
     SF_CUDA(cudaStreamSynchronize(s));
     st->cl_ready = true;
