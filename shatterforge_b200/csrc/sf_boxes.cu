@@ -60,14 +60,16 @@ struct BxArgs {
     uint8_t *wake;
     uint32_t *ent_body, *head;
     int4 *ent_node;          // a grid entry's cell and the next entry of its hash slot
-    uint32_t *cand_a, *cand_b, *hit; float *geom;
+    uint32_t *cand_a, *cand_b, *hit;
     DMan *man[2]; uint64_t *mkey[2]; uint32_t *mcount[2];
     uint32_t *deg, *colour, *corder, *mwait;
     uint2 *mnext;            // per manifold: the next lower priority on each of its bodies
     ulonglong2 *cmask;       // per solver slot: the colours its manifolds took
     float4 *svw;             // per solver slot: velocity, spin
     float4 *sdt;             // per solver slot: the step's translation and rotation so far
-    float4 *sol;             // the manifolds in colour order, BX_SC columns a scene (see SolMan)
+    // the manifolds in colour order, BX_SC columns a scene (see SolMan). Their room, 528 bytes a manifold slot, holds before them
+    // the walk's pairs, the candidates' contact geometry (3,920 bytes a box, of 4,224) and the colouring's lists in turn
+    float4 *sol;
     uint2 *mslot;            // per manifold: its bodies' solver slots
     P3 *sp0; float *sim; DM3 *sii; float4 *sq;
     const uint32_t *sc_b0, *sc_n, *sc_e0, *sc_t0, *sc_tcap, *sc_c0, *sc_m0;   // candidates at c0, manifolds at m0
@@ -320,6 +322,7 @@ __device__ void build_manifold(const BxArgs &A, int par, uint32_t b0, uint32_t s
 // col[j * cap + k]), so that a warp's 32 manifolds are read in whole lines. Read as DMan records, 664 bytes apart, every word
 // of every manifold was a line of its own, some 5,300 of them a warp and pass, which is what bounded the sub-steps.
 // 20,000 boxes, 12 sub-steps on a cluster: 5.48 -> 2.07 ms a step; what is left is the 324 cluster barriers and their latency.
+static_assert((size_t)20 * (BX_PPB + 1) * 4 <= (size_t)BX_CPB * 528, "the contact geometry fits the columns' room");
 enum { SC_N = 0, SC_T1, SC_T2, SC_ID, SC_J, SC_F, SC_E0, SC_CA1, SC_CA2, SC_CB1, SC_CB2, SC_IA1, SC_IA2, SC_IB1, SC_IB2, SC_IAN,
        SC_IBN, SC_P, BX_SC = SC_P + 16 };
 __device__ __forceinline__ float4 f4(P3 a, float w) { return make_float4(a.x, a.y, a.z, w); }
@@ -661,7 +664,8 @@ __global__ void __launch_bounds__(T, CL == 1 && T <= 256 ? 2 : 1) k_box_step(BxA
     // the cell holding the larger of the two minimum corners; then its ground contact (phys.rs:362-365). One walk keeps each
     // body's partners as they come, the counts are scanned, then the lists are written in order; a list of more than BX_SHORT
     // pairs (a static slab under a pile) is sorted by the team, and one that does not fit its row is walked for again.
-    uint32_t *keep = (uint32_t *)(A.geom + (size_t)c0 * 20);
+    float *geom = (float *)(A.sol + (size_t)m0 * BX_SC);
+    uint32_t *keep = (uint32_t *)geom;
     const uint32_t n_ent = GV[G_TOT + 2];            // (a box that counts for entries without having any makes it less than ne_tot)
     walk_pairs(A, b0, e0, n_ent, inv_cell, t, TT, [&](uint32_t a, uint32_t b) {
         const uint32_t k = atomicAdd(&A.cand_n[b0 + a], 1u);
@@ -734,7 +738,7 @@ __global__ void __launch_bounds__(T, CL == 1 && T <= 256 ? 2 : 1) k_box_step(BxA
     if (t == 0) { tm1 = gtime(); tns[0] += tm1 - tm0; tm0 = tm1; }
     // ---- narrow phase, then the manifolds in key order (phys.rs:406-497)
     for (uint32_t c = t; c < nc; c += TT)
-        A.hit[c0 + c] = collide_candidate(A, b0, A.cand_a[c0 + c], A.cand_b[c0 + c], A.geom + (size_t)(c0 + c) * 20) ? 1u : 0u;
+        A.hit[c0 + c] = collide_candidate(A, b0, A.cand_a[c0 + c], A.cand_b[c0 + c], geom + (size_t)c * 20) ? 1u : 0u;
     team_sync<CL>();
     const uint32_t M = team_scan<T, CL>(A.hit + c0, nc, wsum, Gp + G_CTA, t, rank);
     if (M > mcap) {
@@ -743,7 +747,7 @@ __global__ void __launch_bounds__(T, CL == 1 && T <= 256 ? 2 : 1) k_box_step(BxA
     }
     const uint32_t nold = A.mcount[par ^ 1][sc];
     for (uint32_t c = t; c < nc; c += TT) {
-        const float *g = A.geom + (size_t)(c0 + c) * 20;
+        const float *g = geom + (size_t)c * 20;
         const int cnt = __float_as_int(g[3]);
         if (!cnt) continue;
         const uint32_t m = A.hit[c0 + c];
@@ -781,7 +785,7 @@ __global__ void __launch_bounds__(T, CL == 1 && T <= 256 ? 2 : 1) k_box_step(BxA
     }
     team_sync<CL>();
     team_scan<T, CL>(A.deg + s0, ns, wsum, Gp + G_CTA, t, rank);
-    uint64_t *inc = (uint64_t *)(A.geom + (size_t)c0 * 20);      // 2 mcap words of 8 bytes, in the room of the contact geometry (980 n of 4)
+    uint64_t *inc = (uint64_t *)geom;                // 2 mcap words of 8 bytes; the contact geometry is read no more
     for (uint32_t m = t; m < M; m += TT) {
         const uint2 mm = A.mslot[m0 + m];
         const uint64_t ab = A.mkey[par][m0 + m], rk = man_rank((uint32_t)(ab >> 32), (uint32_t)ab, m);
@@ -1004,7 +1008,7 @@ struct sf_box_world {
     DBuf<P3> sp0;
     DBuf<float4> alo, ahi, svw, sdt, sol;
     DBuf<uint2> mslot, mnext;
-    DBuf<float> sim, geom;
+    DBuf<float> sim;
     DBuf<float4> sq;
     DBuf<uint32_t> ecnt, sidx, cand_n, seglong, uf, mint, ent_body, head, cand_a, cand_b, hit, deg, colour,
         corder, mwait, stats, mcount0, mcount1, sc_b0, sc_n, sc_e0, sc_t0, sc_tcap, sc_c0, sc_m0;
@@ -1096,7 +1100,7 @@ extern "C" sf_status sf_box_world_create(const float *boxes, const uint32_t *sce
     A(w->sii.alloc(ns)); A(w->svw.alloc(2 * ns)); A(w->sdt.alloc(2 * ns)); A(w->sol.alloc(mt * BX_SC)); A(w->mslot.alloc(mt)); A(w->sp0.alloc(ns));
     A(w->sim.alloc(ns)); A(w->sq.alloc(ns)); A(w->deg.alloc(ns));
     A(w->ent_body.alloc(et)); A(w->ent_node.alloc(et)); A(w->head.alloc(tt));
-    A(w->cand_a.alloc(ct)); A(w->cand_b.alloc(ct)); A(w->hit.alloc(ct)); A(w->geom.alloc(20 * ct));
+    A(w->cand_a.alloc(ct)); A(w->cand_b.alloc(ct)); A(w->hit.alloc(ct));
     A(w->colour.alloc(mt)); A(w->corder.alloc(mt)); A(w->mwait.alloc(mt)); A(w->mnext.alloc(mt)); A(w->cmask.alloc(ns));
     A(w->man0.alloc(mt)); A(w->man1.alloc(mt)); A(w->mkey0.alloc(mt)); A(w->mkey1.alloc(mt));
     A(w->stats.alloc((size_t)n_scenes * 8)); A(w->tns.alloc((size_t)n_scenes * 5));
@@ -1168,7 +1172,7 @@ extern "C" sf_status sf_box_world_step(sf_box_world *w, float dt, uint32_t nstep
     a.body = w->body.p; a.hulls = w->hulls.p; a.rot = w->rot.p; a.alo = w->alo.p; a.ahi = w->ahi.p;
     a.ecnt = w->ecnt.p; a.sidx = w->sidx.p; a.cand_n = w->cand_n.p; a.seglong = w->seglong.p; a.uf = w->uf.p; a.mint = w->mint.p;
     a.wake = w->wake.p; a.ent_body = w->ent_body.p; a.ent_node = w->ent_node.p; a.head = w->head.p;
-    a.cand_a = w->cand_a.p; a.cand_b = w->cand_b.p; a.hit = w->hit.p; a.geom = w->geom.p;
+    a.cand_a = w->cand_a.p; a.cand_b = w->cand_b.p; a.hit = w->hit.p;
     a.man[0] = w->man0.p; a.man[1] = w->man1.p; a.mkey[0] = w->mkey0.p; a.mkey[1] = w->mkey1.p;
     a.mcount[0] = w->mcount0.p; a.mcount[1] = w->mcount1.p;
     a.deg = w->deg.p; a.colour = w->colour.p; a.corder = w->corder.p; a.mwait = w->mwait.p; a.mnext = w->mnext.p; a.cmask = w->cmask.p;
@@ -1218,10 +1222,11 @@ extern "C" sf_status sf_box_world_read(sf_box_world *w, float *out22) {
     if (!w || !out22) { set_error("null argument"); return SF_ERR_ARG; }
     const uint64_t n22 = (uint64_t)w->n_bodies * 22;
     if (!n22) return SF_OK;
-    // (into the contact geometry's room, free between steps: 980 floats a body)
-    k_box_pack<<<grid_for(n22, 256), 256, 0, w->stream>>>(w->body.p, w->geom.p, n22);
+    // (into the manifold columns' room, free between steps)
+    float *packed = (float *)w->sol.p;
+    k_box_pack<<<grid_for(n22, 256), 256, 0, w->stream>>>(w->body.p, packed, n22);
     SF_CUDA(cudaGetLastError());
-    SF_CUDA(cudaMemcpyAsync(out22, w->geom.p, n22 * sizeof(float), cudaMemcpyDeviceToHost, w->stream));
+    SF_CUDA(cudaMemcpyAsync(out22, packed, n22 * sizeof(float), cudaMemcpyDeviceToHost, w->stream));
     SF_CUDA(cudaStreamSynchronize(w->stream));
     return SF_OK;
 }
