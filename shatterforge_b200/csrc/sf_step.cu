@@ -1342,12 +1342,16 @@ __global__ void k_col_verify(const uint32_t *nm_p, const uint32_t *man_a, const 
 // 7,580 (4) 230 -> 56 us.
 constexpr int SMALL_T = 1024, SMALL_ITEMS = 8;
 constexpr uint32_t SMALL_MAX = SMALL_T * SMALL_ITEMS;
-constexpr uint32_t MASK_DEG = 32;      // manifolds of a body from which its colours are kept as a mask in memory
+constexpr uint32_t MASK_DEG = 32;      // manifolds of a body above which its colours are kept as a mask
 constexpr uint16_t NO_COLOUR = 0xFFFFu;
 constexpr uint32_t SMALL_RANK = 96;    // contacts of a body up to which they are put in order by counting
 // shared memory: sort keys (then each manifold's places in its bodies' lists), priorities, wait counters, the lists,
-// colours, the rounds' queue, contact counts; the colour lists' buckets take the first four once the colours are known
-constexpr size_t SMALL_SMEM = SMALL_MAX * (8 + 4 + 4 + 4 + 2 + 2 + 1);
+// colours, the rounds' queue, contact counts, colour masks; the colour lists' buckets take the first four once the colours
+// are known
+constexpr uint32_t SMALL_MASKS = 6144;   // words of colour masks in shared memory
+constexpr size_t SMALL_SMEM = SMALL_MAX * (8 + 4 + 4 + 4 + 2 + 2 + 1) + SMALL_MASKS * 4;
+constexpr uint32_t SMALL_FEW = 2;        // manifolds of a round that one warp colours
+constexpr uint32_t NO_NEXT = 0x3FFFu;    // (a manifold's number takes 13 bits)
 struct SmallArgs {
     uint32_t nc, nb, K, reduce, max_colors, mw, verify, cstride;
     const uint32_t *L_a, *L_b, *cidx, *body_off;
@@ -1413,7 +1417,8 @@ __global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
     uint16_t *list = (uint16_t *)(wait + SMALL_MAX), *colour = list + 2 * SMALL_MAX;
     uint16_t *queue = colour + SMALL_MAX;
     uint8_t *count = (uint8_t *)(queue + SMALL_MAX);
-    __shared__ uint32_t s_n, s_big, s_ncol, s_queue;
+    uint32_t *smask = (uint32_t *)(count + SMALL_MAX);
+    __shared__ uint32_t s_n, s_big, s_ncol, s_queue, s_lo, s_rounds;
     const uint32_t tid = threadIdx.x;
     if (tid == 0) { s_n = 0; s_big = 0; s_ncol = 0; s_queue = 0; }
     uint32_t nc = A.nc, items = (nc + SMALL_T - 1) / SMALL_T, t0 = tid * items;
@@ -1602,16 +1607,21 @@ __global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
         colour[q] = NO_COLOUR;
     }
     __syncthreads();
+    // The masks lie in shared memory where they fit (else in memory, by body): a list of more than MASK_DEG manifolds is the
+    // only one that starts in its run of MASK_DEG + 1 places.
+    const bool mask_near = (2 * nm / (MASK_DEG + 1) + 1) * A.mw <= SMALL_MASKS;
     auto word = [&](uint32_t c) { return A.nb <= SMALL_MAX ? body[c] : __ldcg(&body[c]); };
 #pragma unroll
     for (int k = 0; k < SMALL_ITEMS; k++) {
         const uint32_t q = tid + k * SMALL_T;
         if (q >= nm) continue;
         auto place = [&](uint32_t c) {
-            const uint32_t n = word(c) & 0xFFFFu;
-            atomicAdd(&body[c], atomicAdd(&s_n, n) << 16);
-            if (n > MASK_DEG)                       // many manifolds at one body: its colours are kept as a mask
-                for (uint32_t i = 0; i < A.mw; i++) A.masks[(size_t)c * A.mw + i] = 0;
+            const uint32_t n = word(c) & 0xFFFFu, s0 = atomicAdd(&s_n, n);
+            atomicAdd(&body[c], s0 << 16);
+            if (n > MASK_DEG) {                     // many manifolds at one body: its colours are kept as a mask
+                uint32_t *mask = mask_near ? smask + s0 / (MASK_DEG + 1) * A.mw : A.masks + (size_t)c * A.mw;
+                for (uint32_t i = 0; i < A.mw; i++) mask[i] = 0;
+            }
         };
         if (pl[4 * q] == 0) place(ca[k]);
         if (cb[k] != STATIC && pl[4 * q + 2] == 0) place(cb[k]);
@@ -1628,33 +1638,63 @@ __global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
         pl[4 * q + 2] = (uint16_t)(wb >> 16); pl[4 * q + 3] = (uint16_t)wb;
     }
     __syncthreads();
-    // a manifold waits for the conflicting ones of higher priority (ties to the lower index)
-    auto before = [&](uint32_t x, uint32_t y) { return prio[x] > prio[y] || (prio[x] == prio[y] && x < y); };
-    // the conflicting manifolds of q that `pick` takes, their list entries and words read four at a time
-    auto conflicts = [&](uint32_t q, auto &&pick_fn, auto &&f) {
+    // A manifold waits for the conflicting ones of higher priority (ties to the lower index): it is coloured once it is the first
+    // uncoloured one at both its bodies. Its word holds at how many bodies another is before it (from bit 28) and the next
+    // lower one at its first (bits 0-13) and second body (14-27): a coloured manifold counts down at most two others, however
+    // many meet at its bodies. Counting down every lower one took a thread n^2 / 2 steps at a hub of n manifolds. This kernel, us,
+    // with that count, with the successors, and the separate launches: 450 manifolds on one body 21,400, 450, 400; 157 2,750,
+    // 173, 180; 774 in a pile on a large body 1,735, 174, 407.
+    for (uint32_t q = tid; q < nm; q += SMALL_T) {
+        const uint32_t mine = prio[q];
+        uint32_t w = 0;
         for (int side = 0; side < 2; side++) {
             const uint32_t s0 = pl[4 * q + 2 * side], n = pl[4 * q + 2 * side + 1];
-            for (uint32_t k = 0; k < n; k += 4) {
-                uint32_t x[4];
-                bool on[4];
+            uint32_t next = NO_NEXT, best = 0;
+            bool higher = false;
+            for (uint32_t k = 0; k < n; k += 4) {   // list entries and words four at a time
+                uint32_t x[4], pr[4];
 #pragma unroll
                 for (int e = 0; e < 4; e++) x[e] = k + e < n ? list[s0 + k + e] : q;
 #pragma unroll
-                for (int e = 0; e < 4; e++) on[e] = x[e] != q && pick_fn(x[e]);
+                for (int e = 0; e < 4; e++) pr[e] = prio[x[e]];
 #pragma unroll
-                for (int e = 0; e < 4; e++) if (on[e]) f(x[e]);
+                for (int e = 0; e < 4; e++) {
+                    if (x[e] == q) continue;
+                    if (pr[e] > mine || (pr[e] == mine && x[e] < q)) higher = true;
+                    else if (next == NO_NEXT || pr[e] > best || (pr[e] == best && x[e] < next)) { next = x[e]; best = pr[e]; }
+                }
             }
+            w |= next << (14 * side);
+            w += higher ? 1u << 28 : 0u;
         }
+        wait[q] = w;
+        if (w >> 28 == 0) queue[atomicAdd(&s_queue, 1u)] = (uint16_t)q;
+    }
+    __syncthreads();
+    // the colour mask of a body with many manifolds, of which q is one: by its list's start in shared memory, else by body
+    auto near_mask = [&](uint32_t s0) { return smask + s0 / (MASK_DEG + 1) * A.mw; };
+    auto far_mask = [&](const uint32_t *man_c, uint32_t q) { return A.masks + (size_t)man_c[q] * A.mw; };
+    const ushort4 *place_of = (const ushort4 *)pl;
+    uint32_t most = 0;
+    // manifold q takes colour c (nothing else of its round is at its bodies)
+    auto take = [&](uint32_t q, ushort4 at, uint32_t c) {
+        if (c >= A.max_colors) { atomicOr(A.err, (unsigned)ERR_CAPACITY_COLORS); c = A.max_colors - 1; }
+        const uint32_t w = wait[q], bit = 1u << (c & 31);
+        colour[q] = (uint16_t)c;
+        if (at.y > MASK_DEG) { if (mask_near) near_mask(at.x)[c >> 5] |= bit; else atomicOr(far_mask(A.man_ca, q) + (c >> 5), bit); }
+        if (at.w > MASK_DEG) { if (mask_near) near_mask(at.z)[c >> 5] |= bit; else atomicOr(far_mask(A.man_cb, q) + (c >> 5), bit); }
+        most = max(most, c + 1);
+        const uint32_t x = w & NO_NEXT, y = (w >> 14) & NO_NEXT;
+        if (x != NO_NEXT && atomicSub(&wait[x], 1u << 28) >> 28 == 1u) queue[atomicAdd(&s_queue, 1u)] = (uint16_t)x;
+        if (y != NO_NEXT && atomicSub(&wait[y], 1u << 28) >> 28 == 1u) queue[atomicAdd(&s_queue, 1u)] = (uint16_t)y;
     };
     // the smallest colour free at both bodies: from the lists' coloured manifolds, or the masks of bodies that keep one
-    auto paint = [&](uint32_t q) {
-        const uint32_t sa = pl[4 * q], na = pl[4 * q + 1], sb = pl[4 * q + 2], nb = pl[4 * q + 3];
-        const uint32_t a = na > MASK_DEG ? A.man_ca[q] : 0u, b = nb > MASK_DEG ? A.man_cb[q] : 0u;
+    auto paint = [&](uint32_t q, ushort4 at) {
         uint32_t c = 0xFFFFFFFFu;
         for (uint32_t k = 0; k < A.mw && c == 0xFFFFFFFFu; k++) {
             uint32_t used = 0;
-            auto gather = [&](uint32_t s0, uint32_t n, uint32_t body_id) {
-                if (n > MASK_DEG) { used |= __ldcg(&A.masks[(size_t)body_id * A.mw + k]); return; }
+            auto gather = [&](uint32_t s0, uint32_t n, const uint32_t *man_c) {
+                if (n > MASK_DEG) { used |= mask_near ? near_mask(s0)[k] : __ldcg(far_mask(man_c, q) + k); return; }
                 for (uint32_t i = 0; i < n; i += 4) {
                     uint32_t x[4];
 #pragma unroll
@@ -1665,52 +1705,84 @@ __global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
                     for (int e = 0; e < 4; e++) if (x[e] >> 5 == k) used |= 1u << (x[e] & 31u);
                 }
             };
-            gather(sa, na, a);
-            gather(sb, nb, b);
+            gather(at.x, at.y, A.man_ca);
+            gather(at.z, at.w, A.man_cb);
             if (~used) c = 32 * k + (__ffs(~used) - 1);
         }
-        if (c >= A.max_colors) { atomicOr(A.err, (unsigned)ERR_CAPACITY_COLORS); c = A.max_colors - 1; }
-        if (na > MASK_DEG) atomicOr(&A.masks[(size_t)a * A.mw + (c >> 5)], 1u << (c & 31));
-        if (nb > MASK_DEG) atomicOr(&A.masks[(size_t)b * A.mw + (c >> 5)], 1u << (c & 31));
         return c;
     };
-    // rounds over a queue: the manifolds that wait for none, then those whose last one was coloured in the round before (few
-    // warps have work in a round, and the others only meet at its barriers)
-    for (uint32_t q = tid; q < nm; q += SMALL_T) {
-        uint32_t n = 0;
-        conflicts(q, [&](uint32_t x) { return before(x, q); }, [&](uint32_t) { n++; });
-        wait[q] = n;
-        if (n == 0) queue[atomicAdd(&s_queue, 1u)] = (uint16_t)q;
-    }
-    __syncthreads();
-    uint32_t rounds = 0, most = 0;
-    for (uint32_t lo = 0, hi = s_queue; lo < hi; rounds++) {
+    // the same by a warp, lane k the mask word k (at most 32) or the k-th entry of a list (at most MASK_DEG): at a hub a round
+    // has few manifolds, and one thread would read the words of its colours one after another
+    static_assert(MAXCOL <= 32 * 32 && MASK_DEG <= 32, "a lane a word and a lane an entry");
+    auto paint_warp = [&](uint32_t q, ushort4 at) -> uint32_t {
+        const uint32_t lane = tid & 31u;
+        uint32_t used = 0;
+        auto gather = [&](uint32_t s0, uint32_t n, const uint32_t *man_c) {
+            if (n > MASK_DEG) { if (lane < A.mw) used |= mask_near ? near_mask(s0)[lane] : __ldcg(far_mask(man_c, q) + lane); return; }
+            const uint32_t own = lane < n ? colour[list[s0 + lane]] : NO_COLOUR;
+            for (uint32_t i = 0; i < n; i++) {
+                const uint32_t x = __shfl_sync(0xffffffffu, own, i);
+                if (x >> 5 == lane) used |= 1u << (x & 31u);
+            }
+        };
+        gather(at.x, at.y, A.man_ca);
+        gather(at.z, at.w, A.man_cb);
+        const uint32_t open = __ballot_sync(0xffffffffu, lane < A.mw && ~used);
+        if (!open) return 0xFFFFFFFFu;
+        const uint32_t k = __ffs(open) - 1;
+        return 32 * k + (__ffs(~__shfl_sync(0xffffffffu, used, k)) - 1);
+    };
+    auto take_warp = [&](uint32_t i) {
+        const uint32_t q = queue[i];
+        const ushort4 at = place_of[q];
+        const uint32_t c = paint_warp(q, at);
+        __syncwarp();
+        if ((tid & 31u) == 0) take(q, at, c);
+        __syncwarp();
+    };
+    // Rounds over a queue: the manifolds that wait for none, then those whose last one was coloured in the round before. Few
+    // warps have work in a round, and the others only meet at its barriers; rounds of a few manifolds, a hub's, go on in one warp
+    // without them.
+    uint32_t rounds = 0;
+    for (uint32_t lo = 0, hi = s_queue; lo < hi;) {
         __syncthreads();
-        for (uint32_t i = lo + tid; i < hi; i += SMALL_T) {
-            const uint32_t q = queue[i], c = paint(q);   // (no conflicting manifold is in the same round)
-            colour[q] = (uint16_t)c;
-            most = max(most, c + 1);
-            for (int side = 0; side < 2; side++) {   // (as conflicts, with the four counters' atomics in flight together)
-                const uint32_t s0 = pl[4 * q + 2 * side], n = pl[4 * q + 2 * side + 1];
-                for (uint32_t k = 0; k < n; k += 4) {
-                    uint32_t x[4], old[4];
-#pragma unroll
-                    for (int e = 0; e < 4; e++) x[e] = k + e < n ? list[s0 + k + e] : q;
-#pragma unroll
-                    for (int e = 0; e < 4; e++) old[e] = x[e] != q && before(q, x[e]) ? atomicSub(&wait[x[e]], 1u) : 0u;
-#pragma unroll
-                    for (int e = 0; e < 4; e++) if (old[e] == 1u) queue[atomicAdd(&s_queue, 1u)] = (uint16_t)x[e];
+        if (hi - lo <= SMALL_FEW) {
+            if (tid < 32) {
+                while (lo < hi && hi - lo <= SMALL_FEW) {
+                    for (; lo < hi; lo++) take_warp(lo);
+                    hi = *(volatile uint32_t *)&s_queue;
+                    rounds++;
                 }
+                if (tid == 0) { s_lo = lo; s_rounds = rounds; }
+            }
+            __syncthreads();
+            lo = s_lo;
+            rounds = s_rounds;
+            hi = s_queue;
+            continue;
+        }
+        if (hi - lo <= SMALL_T / 32) {
+            if (lo + tid / 32 < hi) take_warp(lo + tid / 32);
+        } else {
+            for (uint32_t i = lo + tid; i < hi; i += SMALL_T) {
+                const uint32_t q = queue[i];
+                const ushort4 at = place_of[q];
+                take(q, at, paint(q, at));
             }
         }
         __syncthreads();
         lo = hi;
         hi = s_queue;
+        rounds++;
     }
     atomicMax(&s_ncol, most);
     if (A.verify)
         for (uint32_t q = tid; q < nm; q += SMALL_T)
-            conflicts(q, [&](uint32_t x) { return colour[x] == colour[q]; }, [&](uint32_t) { atomicOr(A.err, (unsigned)ERR_VERIFY_COLOR); });
+            for (int side = 0; side < 2; side++)
+                for (uint32_t k = 0; k < pl[4 * q + 2 * side + 1]; k++) {
+                    const uint32_t x = list[pl[4 * q + 2 * side] + k];
+                    if (x != q && colour[x] == colour[q]) atomicOr(A.err, (unsigned)ERR_VERIFY_COLOR);
+                }
     __syncthreads();
     // colour lists: buckets (colour, contact count descending), then each colour's start and the contact layout
     const uint32_t ncol = s_ncol, nb = ncol * JDS_ROW;
