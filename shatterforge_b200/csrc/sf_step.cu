@@ -26,6 +26,7 @@
 //   k_integrate      pinch clamps (src/lib.rs:1746-1768) and integrate (src/lib.rs:1703-1742)
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "sf_internal.cuh"
 
@@ -1905,10 +1906,12 @@ __device__ __forceinline__ Contact load_contact(const SolveArgs &A, uint32_t at)
 }
 // solve() of one contact (src/lib.rs:1579-1601); its new impulses are returned. STRAIGHT computes the second body's side
 // without branches also where there is none (zero mass and arms; its velocity at the contact is then replaced by 0), so
-// that the two sides' chains interleave: a lane of a small substep is alone on its scheduler.
-template <bool STRAIGHT>
+// that the two sides' chains interleave: a lane of a small substep is alone on its scheduler. NO_SECOND leaves it out.
+enum Sides { BRANCH, STRAIGHT_BOTH, NO_SECOND };
+template <Sides SIDES>
 __device__ __forceinline__ float4 solve_contact(Pair &P, const Contact &c) {
-    const bool hasb = P.hasb;
+    constexpr bool STRAIGHT = SIDES == STRAIGHT_BOTH;
+    const bool hasb = SIDES != NO_SECOND && P.hasb;
     float4 j4 = c.j;
     const V3 n = v3(c.n.x, c.n.y, c.n.z), t1 = v3(c.t1.x, c.t1.y, c.t1.z), t2 = v3(c.t2.x, c.t2.y, c.t2.z);
     const V3 ra = v3(c.ra.x, c.ra.y, c.ra.z), rb = v3(c.rb.x, c.rb.y, c.rb.z);
@@ -1959,7 +1962,7 @@ __device__ __forceinline__ void solve_manifold(const SolveArgs &A, uint32_t i, u
         const Contact c = nx;
         if (k + 1 < P.cnt) nx = load_contact<false>(A, off[k + 1] + p);
         if (warm) warm_contact(P, c);
-        else A.S_j[off[k] + p] = solve_contact<false>(P, c);
+        else A.S_j[off[k] + p] = solve_contact<BRANCH>(P, c);
     }
     store_vel(A, P);
 }
@@ -1999,18 +2002,25 @@ __global__ void __launch_bounds__(SOLVE_BLOCK) k_solve(SolveArgs A) {
 }
 
 // Small substeps (at most SOLVE_TEAM_MAX contacts): one block (NB = 1), or one cluster of NB blocks, with everything the
-// iterations touch in shared memory: the active bodies' velocities (body t in block t % NB) and the contacts (position p
-// of a colour in block p % NB). What bounds a colour pass there is the chain of its longest manifold, up to 32 contacts of
-// some 300 dependent-issue operations; read from L2 a contact took 780 to 930 cycles, the latency of its six words.
+// iterations touch in shared memory: the active bodies' velocities (body t in block t % NB), the contacts (position p
+// of colour c in block (p + c) % NB, so that colours of one manifold, a large body's, fill all the blocks) and the places of
+// both. What bounds a colour pass there is the chain of its longest manifold, up to 32 contacts of some 300 dependent-issue
+// operations; read from L2 a contact took 780 to 930 cycles, the latency of its six words.
 // Solve of 8 iterations, against one block (or warp) that read everything through L1: 1,300 contacts 140 -> 107 us (alone;
-// 114 on the cluster), 2,980 198 -> 143 us, 3,600 242 -> 133 us, 7,580 288 -> 147 us. A contact now takes 590 cycles, about
-// its instructions at one every two cycles of the one warp that runs the chain.
+// 114 on the cluster), 2,980 198 -> 143 us, 3,600 242 -> 133 us, 7,580 288 -> 147 us. A contact then took 590 cycles, about
+// its instructions at one every two cycles of the one warp that runs the chain. One body on the ground, whose colours are a
+// manifold each, ms: 576 contacts 1.33 -> 1.14 (470 cycles a contact without the second body's side), 2,500 6.83 -> 4.23, 7,200
+// 22.4 -> 12.2; with places for 64 colours only and every such colour in block 0, these took 1.50, 8.9 and 25.4.
 constexpr int SOLVE_TEAM_BLOCKS = 16, SOLVE_TEAM_T = 128, SOLVE_TEAM_T1 = 256;   // threads a block of the cluster / alone
 constexpr uint32_t SOLVE_TEAM_MAX = 8192;          // contacts
 constexpr uint32_t SMALL_SUBSTEP_CONTACTS = 1024;  // contacts up to which the colouring runs on one block
-constexpr uint32_t SOLVE_TEAM_COLS = 64;           // colours whose tables are kept in shared memory
-constexpr uint32_t SOLVE_TEAM_SMEM = 196 * 1024;
+constexpr uint32_t SOLVE_TEAM_ROWS = 16384;        // rows (colour, k) whose places are kept in shared memory
+constexpr uint32_t SOLVE_TEAM_SMEM = 224 * 1024, SOLVE_TEAM_ALONE = 196 * 1024;   // bytes a block; up to which one is alone
 constexpr uint32_t SOLVE_TEAM_BODIES = 4096;       // bodies a block
+// bytes of the places: two tables of the rows (alone one) and the colours' starts
+static uint32_t solve_team_places(uint32_t rows, uint32_t K, bool alone) {
+    return (2 * ((rows + 1) * (alone ? 1 : 2) + rows / K + 2) + 15) / 16 * 16;
+}
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t a) {
     float4 v;
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
@@ -2023,27 +2033,33 @@ __device__ __forceinline__ void cp_async16(float4 *to, const float4 *from) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from) : "memory");
 }
 template <int NB, int T>
-__global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *nc_p, uint32_t slots) {
-    extern __shared__ float4 sv[];                 // velocity, spin of bodies rank, rank + NB, ...; then the contacts
-    __shared__ uint32_t s_start[SOLVE_TEAM_COLS + 1], s_off[SOLVE_TEAM_COLS * JDS_K + 1], s_loc[SOLVE_TEAM_COLS * JDS_K + 1];
+__global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *nc_p, uint32_t K, uint32_t slots, uint32_t max_rows) {
+    static_assert((NB & (NB - 1)) == 0, "a power of two");
+    extern __shared__ float4 sv[];                 // velocity, spin of bodies rank, rank + NB, ...; the contacts; the places
     __shared__ uint32_t s_base[NB];                // shared::cluster address of every block's velocities
     __shared__ uint32_t s_sum[T / 32];
-    const uint32_t rank = blockIdx.x, g = threadIdx.x * NB + rank, lane = threadIdx.x & 31;
+    const uint32_t rank = blockIdx.x, lane = threadIdx.x & 31;
     constexpr uint32_t stride = NB * T;
-    const uint32_t ncol = A.dev[DV_COLORS], rows = ncol * JDS_K;
-    const bool tab = ncol <= SOLVE_TEAM_COLS;
+    const uint32_t ncol = A.dev[DV_COLORS], rows = ncol * K;   // (a manifold has at most K contacts)
+    const bool tab = rows <= max_rows;
     const uint32_t nbl = (A.nb + NB - 1) / NB;
     float4 *sc = sv + 2 * nbl;                     // six columns of `slots` contacts
-    uint32_t used = 0;
+    uint16_t *s_off = (uint16_t *)(sc + 6 * (size_t)slots), *s_start = s_off + max_rows + 1;
+    uint16_t *s_loc = NB == 1 ? s_off : s_start + max_rows / K + 2;   // (a block alone keeps the contacts in their places)
+    // the first position of colour c in this block
+    auto first = [&](uint32_t c) { return (rank - c) & (NB - 1); };
+    uint32_t used = NB == 1 ? *nc_p : 0u;
     if (tab) {
-        for (uint32_t k = threadIdx.x; k <= ncol; k += T) s_start[k] = A.col_start[k];
-        for (uint32_t k = threadIdx.x; k <= rows; k += T) s_off[k] = k < rows ? A.jds_off[k] : *nc_p;
+        for (uint32_t k = threadIdx.x; k <= ncol; k += T) s_start[k] = (uint16_t)A.col_start[k];
+        for (uint32_t k = threadIdx.x; k <= rows; k += T) s_off[k] = (uint16_t)(k < rows ? A.jds_off[k / K * JDS_K + k % K] : *nc_p);
         __syncthreads();
-        // row (colour, k): the k-th contacts of the colour's manifolds, n of them; those of this block are positions
-        // rank, rank + NB, ... and go to consecutive slots
+    }
+    if (NB > 1 && tab) {
+        // row (colour c, k): the k-th contacts of the colour's manifolds, n of them; those of this block are positions
+        // first(c), first(c) + NB, ... and go to consecutive slots
         for (uint32_t r0 = 0; r0 < rows; r0 += T) {
-            const uint32_t r = r0 + threadIdx.x, n = r < rows ? s_off[r + 1] - s_off[r] : 0u;
-            const uint32_t m = n > rank ? (n - rank + NB - 1) / NB : 0u;
+            const uint32_t r = r0 + threadIdx.x, n = r < rows ? (uint32_t)s_off[r + 1] - s_off[r] : 0u, p0 = first(r / K);
+            const uint32_t m = n > p0 ? (n - p0 + NB - 1) / NB : 0u;
             uint32_t x = m;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= (uint32_t)o) x += y; }
@@ -2051,21 +2067,26 @@ __global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *n
             __syncthreads();
             uint32_t before = used, all = 0;
             for (uint32_t w = 0; w < T / 32; w++) { if (w < threadIdx.x >> 5) before += s_sum[w]; all += s_sum[w]; }
-            if (r < rows) s_loc[r] = before + x - m;
+            if (r < rows) s_loc[r] = (uint16_t)(before + x - m);
             used += all;
             __syncthreads();
         }
-        if (threadIdx.x == 0) s_loc[rows] = used;
+        if (threadIdx.x == 0) s_loc[rows] = (uint16_t)used;
         __syncthreads();
     }
     const bool resident = tab && used <= slots;    // else the contacts are read from memory
-    const uint32_t *start = tab ? s_start : A.col_start, *offs = tab ? s_off : A.jds_off;
     // the slots, in runs of one row: thread by thread over all of them
     auto each_slot = [&](auto &&f) {
         uint32_t r = 0;
         for (uint32_t q = threadIdx.x; q < used; q += T) {
-            while (s_loc[r + 1] <= q) r++;
-            f(q, (size_t)s_off[r] + rank + (q - s_loc[r]) * NB);
+            if constexpr (NB == 1) f(q, q);
+            else {
+                for (uint32_t hi = rows; hi - r > 1;) {   // the row that holds slot q: the last one that begins at or before it
+                    const uint32_t mid = (r + hi) >> 1;
+                    if (s_loc[mid] <= q) r = mid; else hi = mid;
+                }
+                f(q, (size_t)s_off[r] + first(r / K) + (q - s_loc[r]) * NB);
+            }
         }
     };
     if (resident)
@@ -2106,23 +2127,25 @@ __global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *n
         if (NB == 1) { sv[2 * t] = make_float4(v.x, v.y, v.z, 0.0f); sv[2 * t + 1] = make_float4(w.x, w.y, w.z, 0.0f); }
         else { const uint32_t at = s_base[t % NB] + (t / NB) * 32u; st_cluster_v3(at, v); st_cluster_v3(at + 16, w); }
     };
-    // this thread's manifolds: for each iteration and colour, the positions g, g + stride, ...; the next one's bodies and
+    // this thread's manifolds: for each iteration and colour, its position of each round of `stride`; the next one's bodies and
     // masses are loaded while the current one is solved
-    uint32_t c = 0, p = g, it = 0;
+    uint32_t c = 0, round = 0, it = 0;
     const uint32_t iters = ncol ? A.iterations + A.warm : 0u;
+    auto start = [&](uint32_t k) -> uint32_t { return tab ? s_start[k] : A.col_start[k]; };
+    auto position = [&]() { return round + threadIdx.x * NB + first(c); };
     Pair nx;
     auto prefetch = [&]() {
         nx.cnt = 0;
-        if (it < iters && p < start[c + 1] - start[c]) nx = load_pair(A, start[c] + p);
+        if (it < iters && position() < start(c + 1) - start(c)) nx = load_pair(A, start(c) + position());
     };
     prefetch();
     while (it < iters) {
-        const uint32_t c0 = c, p0 = p;
+        const uint32_t c0 = c, p0 = position();
         const bool warm = A.warm && it == 0;
-        const bool last = p - g + stride >= start[c + 1] - start[c];   // the colour's last round
-        p += stride;
+        const bool last = round + stride >= start(c + 1) - start(c);   // the colour's last round
+        round += stride;
         if (last) {
-            p = g;
+            round = 0;
             if (++c == ncol) { c = 0; it++; }
         }
         Pair P = nx;
@@ -2133,30 +2156,43 @@ __global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *n
             if (P.hasb) load_v(P.b, P.vb, P.wb);
         }
         prefetch();
+        // a warp whose manifolds are all against the ground or static bodies leaves the second side out
+        const bool two = __any_sync(0xffffffffu, P.cnt && P.hasb);
         if (P.cnt) {
-            const uint32_t *off = offs + c0 * JDS_K;
-            if (resident) {
-                const uint32_t *loc = s_loc + c0 * JDS_K, lp = p0 / NB;
-                auto get = [&](uint32_t q) {
-                    Contact x;
-                    x.n = sc[q]; x.t1 = sc[slots + q]; x.t2 = sc[2 * slots + q]; x.ra = sc[3 * slots + q]; x.rb = sc[4 * slots + q];
-                    x.j = sc[5 * slots + q];
-                    return x;
-                };
-                Contact y = get(loc[0] + lp);
-                for (uint32_t k = 0; k < P.cnt; k++) {
-                    const Contact x = y;
-                    if (k + 1 < P.cnt) y = get(loc[k + 1] + lp);
-                    if (warm) warm_contact(P, x);
-                    else sc[5 * slots + loc[k] + lp] = solve_contact<true>(P, x);
+            auto chain = [&](auto sides) {
+                constexpr Sides SIDES = decltype(sides)::value;
+                if (resident) {
+                    const uint16_t *loc = s_loc + c0 * K;
+                    const uint32_t lp = p0 / NB;
+                    auto get = [&](uint32_t q) {
+                        Contact x;
+                        x.n = sc[q]; x.t1 = sc[slots + q]; x.t2 = sc[2 * slots + q]; x.ra = sc[3 * slots + q]; x.rb = sc[4 * slots + q];
+                        x.j = sc[5 * slots + q];
+                        return x;
+                    };
+                    uint32_t at = loc[0] + lp;
+                    Contact y = get(at);
+                    for (uint32_t k = 0; k < P.cnt; k++) {
+                        const Contact x = y;
+                        const uint32_t own = at;
+                        if (k + 1 < P.cnt) { at = loc[k + 1] + lp; y = get(at); }
+                        if (warm) warm_contact(P, x);
+                        else sc[5 * slots + own] = solve_contact<SIDES>(P, x);
+                    }
+                } else {
+                    const uint32_t *off = A.jds_off + c0 * JDS_K;
+                    uint32_t at = off[0] + p0;
+                    Contact y = load_contact<true>(A, at);
+                    for (uint32_t k = 0; k < P.cnt; k++) {
+                        const Contact x = y;
+                        const uint32_t own = at;
+                        if (k + 1 < P.cnt) { at = off[k + 1] + p0; y = load_contact<true>(A, at); }
+                        if (warm) warm_contact(P, x);
+                        else A.S_j[own] = solve_contact<SIDES>(P, x);
+                    }
                 }
-            } else {
-                for (uint32_t k = 0; k < P.cnt; k++) {
-                    const Contact x = load_contact<true>(A, off[k] + p0);
-                    if (warm) warm_contact(P, x);
-                    else A.S_j[off[k] + p0] = solve_contact<true>(P, x);
-                }
-            }
+            };
+            if (two) chain(std::integral_constant<Sides, STRAIGHT_BOTH>{}); else chain(std::integral_constant<Sides, NO_SECOND>{});
             store_v(P.a, P.va, P.wa);
             if (P.hasb) store_v(P.b, P.vb, P.wb);
         }
@@ -3046,14 +3082,17 @@ static sf_status substep(sf_world *w, float h) {
         A.vw = S->vw.p; A.nb = nb; A.gb = S->dom_gb.p; A.err = w->err.p;
         A.warm = w->P.warm_start ? 1u : 0u;
         if (one_block) {
-            // alone a block holds the contacts of about 1,500 (SOLVE_TEAM_SMEM, 96 bytes each beside its bodies)
-            const bool alone = !S->team_ok || (uint64_t)nb * 32 + (uint64_t)ncm * 96 <= SOLVE_TEAM_SMEM;
+            // alone a block holds the contacts of about 1,500 (SOLVE_TEAM_ALONE, 96 bytes each beside its bodies)
+            const bool alone = !S->team_ok || (uint64_t)nb * 32 + (uint64_t)ncm * 96 <= SOLVE_TEAM_ALONE;
             const uint32_t nbl = alone ? nb : (nb + SOLVE_TEAM_BLOCKS - 1) / SOLVE_TEAM_BLOCKS;
-            // a block's contacts: an even share of each row (colour, k), rounded up
-            const uint32_t want = alone ? ncm : ncm / SOLVE_TEAM_BLOCKS + SOLVE_TEAM_COLS * JDS_K;
-            const uint32_t slots = std::min(want, (SOLVE_TEAM_SMEM - nbl * 32) / 96);
-            const size_t smem = (size_t)nbl * 32 + (size_t)slots * 96;
-            if (alone) k_solve_team<1, SOLVE_TEAM_T1><<<1, SOLVE_TEAM_T1, smem, s>>>(A, S->dev.p + DV_KEPT, slots);
+            // as many rows as the colours can have, while they leave room for the contacts
+            const uint32_t K = w->P.manifold_chunk;
+            const uint32_t max_rows = (uint32_t)std::min<uint64_t>((uint64_t)std::min(w->P.max_colors, ncm) * K, SOLVE_TEAM_ROWS);
+            const uint32_t places = solve_team_places(max_rows, K, alone);
+            // (a block takes no more contacts than there are)
+            const uint32_t slots = std::min(ncm, (SOLVE_TEAM_SMEM - std::min(SOLVE_TEAM_SMEM, nbl * 32 + places)) / 96);
+            const size_t smem = (size_t)nbl * 32 + (size_t)slots * 96 + places;
+            if (alone) k_solve_team<1, SOLVE_TEAM_T1><<<1, SOLVE_TEAM_T1, smem, s>>>(A, S->dev.p + DV_KEPT, K, slots, max_rows);
             else {
                 cudaLaunchConfig_t cfg = {};
                 cudaLaunchAttribute at[1];
@@ -3066,7 +3105,7 @@ static sf_status substep(sf_world *w, float h) {
                 cfg.attrs = at;
                 cfg.numAttrs = 1;
                 SF_CUDA(cudaLaunchKernelEx(&cfg, k_solve_team<SOLVE_TEAM_BLOCKS, SOLVE_TEAM_T>, A,
-                                           (const uint32_t *)(S->dev.p + DV_KEPT), slots));
+                                           (const uint32_t *)(S->dev.p + DV_KEPT), K, slots, max_rows));
             }
         } else {
             SF_CUDA(cudaMemsetAsync(S->dom_gb.p, 0, (size_t)S->part_D * sizeof(GridBarrier), s));
