@@ -1345,6 +1345,9 @@ constexpr int SMALL_T = 1024, SMALL_ITEMS = 8;
 constexpr uint32_t SMALL_MAX = SMALL_T * SMALL_ITEMS;
 constexpr uint32_t MASK_DEG = 32;      // manifolds of a body above which its colours are kept as a mask
 constexpr uint16_t NO_COLOUR = 0xFFFFu;
+// a sort key: the pair's first body from bit 38, its second (0 for none) from bit 13, the contact's place in the list
+constexpr int KEY_A = 38, KEY_B = 13;
+constexpr uint32_t SMALL_BODIES = (1u << (KEY_A - KEY_B)) - 1;   // active bodies at most
 constexpr uint32_t SMALL_RANK = 96;    // contacts of a body up to which they are put in order by counting
 // shared memory: sort keys (then each manifold's places in its bodies' lists), priorities, wait counters, the lists,
 // colours, the rounds' queue, contact counts, colour masks; the colour lists' buckets take the first four once the colours
@@ -1435,12 +1438,12 @@ __global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
         for (int k = 0; k < SMALL_ITEMS; k++) {
             const uint32_t t = tid + k * SMALL_T;
             if (t < nc)
-                key[t] = ((unsigned long long)A.cidx[la[k]] << 30) |
-                         ((unsigned long long)(lb[k] == STATIC ? 0u : A.cidx[lb[k]] + 1) << 13) | t;
+                key[t] = ((unsigned long long)A.cidx[la[k]] << KEY_A) |
+                         ((unsigned long long)(lb[k] == STATIC ? 0u : A.cidx[lb[k]] + 1) << KEY_B) | t;
         }
     }
     __syncthreads();
-    // each thread's run of contacts, t0 .. t0 + items, and where the body (drop = 30) or pair (13) of each begins
+    // each thread's run of contacts, t0 .. t0 + items, and where the body (drop = KEY_A) or pair (KEY_B) of each begins
     uint32_t begin[SMALL_ITEMS];
     auto begins = [&](int drop) {
         uint32_t own = 0;                           // the last place in the run where one begins, + 1
@@ -1457,7 +1460,7 @@ __global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
     // Contacts by (a, b), each pair's in list order. The list comes in the bricks' order and a body's bricks lie together,
     // so as a rule it only has to be put in order within each body: a contact's place is the number of smaller keys among
     // its body's. A body with many contacts, or bodies out of order, take the whole sort.
-    begins(30);
+    begins(KEY_A);
     {
         unsigned long long own[SMALL_ITEMS];
         uint32_t to[SMALL_ITEMS];
@@ -1467,9 +1470,9 @@ __global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
             const uint32_t t = t0 + k;
             if (k >= (int)items || t >= nc) continue;
             own[k] = key[t];
-            if (t && (key[t - 1] >> 30) > (own[k] >> 30)) bad = true;
+            if (t && (key[t - 1] >> KEY_A) > (own[k] >> KEY_A)) bad = true;
             // four at a time, past the body's end too (a larger body's keys are not smaller)
-            const unsigned long long body_end = ((own[k] >> 30) + 1) << 30;
+            const unsigned long long body_end = ((own[k] >> KEY_A) + 1) << KEY_A;
             uint32_t u = begin[k], less = 0;
             for (bool more = true; more && u < begin[k] + SMALL_RANK; u += 4) {
                 unsigned long long x[4];
@@ -1495,7 +1498,7 @@ __global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
             __syncthreads();
         }
     }
-    begins(13);
+    begins(KEY_B);
     if (A.reduce) {
         // contact reduction (see RED_K above): a pair's contacts counted at its first place, which `first` gives
         uint16_t *first = colour;
@@ -1549,7 +1552,7 @@ __global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
             items = (nc + SMALL_T - 1) / SMALL_T;
             t0 = tid * items;
             __syncthreads();
-            begins(13);
+            begins(KEY_B);
         }
     }
     // chunks of K: the manifolds, in (a, b) order; each one's first contact, then its words
@@ -1585,8 +1588,8 @@ __global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
         const uint32_t a = A.L_a[c], b = A.L_b[c], off = A.body_off[a];
         const uint32_t h = pair_priority(a - off, b == STATIC ? 0u : b - off + 1u);
         const uint32_t pr = j ? pair_priority(h, j) : h;
-        ca[k] = (uint32_t)(key[t] >> 30);
-        if (b != STATIC) cb[k] = (uint32_t)(key[t] >> 13 & 0x1FFFFu) - 1u;
+        ca[k] = (uint32_t)(key[t] >> KEY_A);
+        if (b != STATIC) cb[k] = (uint32_t)(key[t] >> KEY_B & SMALL_BODIES) - 1u;
         A.man_a[q] = a; A.man_b[q] = b; A.man_ca[q] = ca[k]; A.man_cb[q] = cb[k];
         A.man_start[q] = t; A.man_count[q] = n; A.man_prio[q] = pr;
         prio[q] = pr;
@@ -2016,7 +2019,7 @@ constexpr uint32_t SOLVE_TEAM_MAX = 8192;          // contacts
 constexpr uint32_t SMALL_SUBSTEP_CONTACTS = 1024;  // contacts up to which the colouring runs on one block
 constexpr uint32_t SOLVE_TEAM_ROWS = 16384;        // rows (colour, k) whose places are kept in shared memory
 constexpr uint32_t SOLVE_TEAM_SMEM = 224 * 1024, SOLVE_TEAM_ALONE = 196 * 1024;   // bytes a block; up to which one is alone
-constexpr uint32_t SOLVE_TEAM_BODIES = 4096;       // bodies a block
+constexpr uint32_t SOLVE_TEAM_BODIES = 4096;       // bodies a block; of more the velocities stay in memory
 // bytes of the places: two tables of the rows (alone one) and the colours' starts
 static uint32_t solve_team_places(uint32_t rows, uint32_t K, bool alone) {
     return (2 * ((rows + 1) * (alone ? 1 : 2) + rows / K + 2) + 15) / 16 * 16;
@@ -2032,7 +2035,10 @@ __device__ __forceinline__ void st_cluster_v3(uint32_t a, V3 v) {
 __device__ __forceinline__ void cp_async16(float4 *to, const float4 *from) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from) : "memory");
 }
-template <int NB, int T>
+// NEAR: the velocities lie in shared memory. Worlds of more bodies than fit there read and write them in memory: alone through
+// L1, a cluster through L2 (its barriers order them). A step of 80,000 bodies of which 100 lie in a heap (180 contacts) takes 0.61
+// ms so; with the kernels of large substeps it took 1.24, with the former one-block solve and separate launches 1.03.
+template <int NB, int T, bool NEAR>
 __global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *nc_p, uint32_t K, uint32_t slots, uint32_t max_rows) {
     static_assert((NB & (NB - 1)) == 0, "a power of two");
     extern __shared__ float4 sv[];                 // velocity, spin of bodies rank, rank + NB, ...; the contacts; the places
@@ -2042,7 +2048,7 @@ __global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *n
     constexpr uint32_t stride = NB * T;
     const uint32_t ncol = A.dev[DV_COLORS], rows = ncol * K;   // (a manifold has at most K contacts)
     const bool tab = rows <= max_rows;
-    const uint32_t nbl = (A.nb + NB - 1) / NB;
+    const uint32_t nbl = NEAR ? (A.nb + NB - 1) / NB : 0u;
     float4 *sc = sv + 2 * nbl;                     // six columns of `slots` contacts
     uint16_t *s_off = (uint16_t *)(sc + 6 * (size_t)slots), *s_start = s_off + max_rows + 1;
     uint16_t *s_loc = NB == 1 ? s_off : s_start + max_rows / K + 2;   // (a block alone keeps the contacts in their places)
@@ -2077,7 +2083,7 @@ __global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *n
     const bool resident = tab && used <= slots;    // else the contacts are read from memory
     // the slots, in runs of one row: thread by thread over all of them
     auto each_slot = [&](auto &&f) {
-        uint32_t r = 0;
+        [[maybe_unused]] uint32_t r = 0;
         for (uint32_t q = threadIdx.x; q < used; q += T) {
             if constexpr (NB == 1) f(q, q);
             else {
@@ -2098,7 +2104,7 @@ __global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *n
             cp_async16(&sc[4 * slots + q], &A.S_rb[at]);
             cp_async16(&sc[5 * slots + q], &A.S_j[at]);
         });
-    for (uint32_t k = threadIdx.x; k * NB + rank < A.nb; k += T) {
+    for (uint32_t k = threadIdx.x; NEAR && k * NB + rank < A.nb; k += T) {
         const size_t t = (size_t)k * NB + rank;
         cp_async16(&sv[2 * k], &A.vw[2 * t]);
         cp_async16(&sv[2 * k + 1], &A.vw[2 * t + 1]);
@@ -2118,13 +2124,19 @@ __global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *n
     sync();
     auto load_v = [&](uint32_t t, V3 &v, V3 &w) {
         float4 a, b;
-        if (NB == 1) { a = sv[2 * t]; b = sv[2 * t + 1]; }
+        const float4 *far = A.vw + 2 * (size_t)t;
+        if (!NEAR) { a = NB == 1 ? far[0] : __ldcg(far); b = NB == 1 ? far[1] : __ldcg(far + 1); }
+        else if (NB == 1) { a = sv[2 * t]; b = sv[2 * t + 1]; }
         else { const uint32_t at = s_base[t % NB] + (t / NB) * 32u; a = ld_cluster_f4(at); b = ld_cluster_f4(at + 16); }
         v = v3(a.x, a.y, a.z);
         w = v3(b.x, b.y, b.z);
     };
     auto store_v = [&](uint32_t t, V3 v, V3 w) {
-        if (NB == 1) { sv[2 * t] = make_float4(v.x, v.y, v.z, 0.0f); sv[2 * t + 1] = make_float4(w.x, w.y, w.z, 0.0f); }
+        if (!NEAR || NB == 1) {
+            float4 *at = (NEAR ? sv : A.vw) + 2 * (size_t)t;
+            at[0] = make_float4(v.x, v.y, v.z, 0.0f);
+            at[1] = make_float4(w.x, w.y, w.z, 0.0f);
+        }
         else { const uint32_t at = s_base[t % NB] + (t / NB) * 32u; st_cluster_v3(at, v); st_cluster_v3(at + 16, w); }
     };
     // this thread's manifolds: for each iteration and colour, its position of each round of `stride`; the next one's bodies and
@@ -2200,7 +2212,7 @@ __global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *n
     }
     sync();
     if (resident) each_slot([&](uint32_t q, size_t at) { A.S_j[at] = sc[5 * slots + q]; });
-    for (uint32_t k = threadIdx.x; k * NB + rank < A.nb; k += T) {
+    for (uint32_t k = threadIdx.x; NEAR && k * NB + rank < A.nb; k += T) {
         const size_t t = (size_t)k * NB + rank;
         A.vw[2 * t] = sv[2 * k];
         A.vw[2 * t + 1] = sv[2 * k + 1];
@@ -2612,11 +2624,10 @@ sf_status step_create(sf_world *w) {
     SF_CUDA(grow_contacts(S, initial));
     int occ = 0;
     {
-        auto *one = k_solve_team<1, SOLVE_TEAM_T1>;
-        auto *team = k_solve_team<SOLVE_TEAM_BLOCKS, SOLVE_TEAM_T>;
-        SF_CUDA(cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLVE_TEAM_SMEM));
-        SF_CUDA(cudaFuncSetAttribute(team, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLVE_TEAM_SMEM));
-        SF_CUDA(cudaFuncSetAttribute(team, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        auto *team = k_solve_team<SOLVE_TEAM_BLOCKS, SOLVE_TEAM_T, true>, *team_far = k_solve_team<SOLVE_TEAM_BLOCKS, SOLVE_TEAM_T, false>;
+        for (auto *k : {k_solve_team<1, SOLVE_TEAM_T1, true>, k_solve_team<1, SOLVE_TEAM_T1, false>, team, team_far})
+            SF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLVE_TEAM_SMEM));
+        for (auto *k : {team, team_far}) SF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchConfig_t c = {};
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -2897,7 +2908,7 @@ static sf_status substep(sf_world *w, float h) {
     prof_mark(w);
     // The launch size of the colouring and the solve, and its partition into sync domains. A substep with few contacts
     // is solved by one block or cluster (k_solve_team); its colouring then runs as a single domain.
-    const bool one_block = nc <= SOLVE_TEAM_MAX && nb <= (S->team_ok ? SOLVE_TEAM_BLOCKS : 1) * SOLVE_TEAM_BODIES;
+    const bool one_block = nc <= SOLVE_TEAM_MAX && nb <= SMALL_BODIES;
     int sci = -1;
     const int sb = Tuner::bucket(nc);
     const unsigned top_occ = (unsigned)std::min(S->solve_occ, S->jp_occ);
@@ -3083,8 +3094,9 @@ static sf_status substep(sf_world *w, float h) {
         A.warm = w->P.warm_start ? 1u : 0u;
         if (one_block) {
             // alone a block holds the contacts of about 1,500 (SOLVE_TEAM_ALONE, 96 bytes each beside its bodies)
-            const bool alone = !S->team_ok || (uint64_t)nb * 32 + (uint64_t)ncm * 96 <= SOLVE_TEAM_ALONE;
-            const uint32_t nbl = alone ? nb : (nb + SOLVE_TEAM_BLOCKS - 1) / SOLVE_TEAM_BLOCKS;
+            const bool far = nb > (S->team_ok ? SOLVE_TEAM_BLOCKS : 1) * SOLVE_TEAM_BODIES;
+            const bool alone = !S->team_ok || (far ? 0 : (uint64_t)nb * 32) + (uint64_t)ncm * 96 <= SOLVE_TEAM_ALONE;
+            const uint32_t nbl = far ? 0u : alone ? nb : (nb + SOLVE_TEAM_BLOCKS - 1) / SOLVE_TEAM_BLOCKS;
             // as many rows as the colours can have, while they leave room for the contacts
             const uint32_t K = w->P.manifold_chunk;
             const uint32_t max_rows = (uint32_t)std::min<uint64_t>((uint64_t)std::min(w->P.max_colors, ncm) * K, SOLVE_TEAM_ROWS);
@@ -3092,7 +3104,10 @@ static sf_status substep(sf_world *w, float h) {
             // (a block takes no more contacts than there are)
             const uint32_t slots = std::min(ncm, (SOLVE_TEAM_SMEM - std::min(SOLVE_TEAM_SMEM, nbl * 32 + places)) / 96);
             const size_t smem = (size_t)nbl * 32 + (size_t)slots * 96 + places;
-            if (alone) k_solve_team<1, SOLVE_TEAM_T1><<<1, SOLVE_TEAM_T1, smem, s>>>(A, S->dev.p + DV_KEPT, K, slots, max_rows);
+            if (alone) {
+                if (far) k_solve_team<1, SOLVE_TEAM_T1, false><<<1, SOLVE_TEAM_T1, smem, s>>>(A, S->dev.p + DV_KEPT, K, slots, max_rows);
+                else k_solve_team<1, SOLVE_TEAM_T1, true><<<1, SOLVE_TEAM_T1, smem, s>>>(A, S->dev.p + DV_KEPT, K, slots, max_rows);
+            }
             else {
                 cudaLaunchConfig_t cfg = {};
                 cudaLaunchAttribute at[1];
@@ -3104,7 +3119,7 @@ static sf_status substep(sf_world *w, float h) {
                 cfg.stream = s;
                 cfg.attrs = at;
                 cfg.numAttrs = 1;
-                SF_CUDA(cudaLaunchKernelEx(&cfg, k_solve_team<SOLVE_TEAM_BLOCKS, SOLVE_TEAM_T>, A,
+                SF_CUDA(cudaLaunchKernelEx(&cfg, far ? k_solve_team<SOLVE_TEAM_BLOCKS, SOLVE_TEAM_T, false> : k_solve_team<SOLVE_TEAM_BLOCKS, SOLVE_TEAM_T, true>, A,
                                            (const uint32_t *)(S->dev.p + DV_KEPT), K, slots, max_rows));
             }
         } else {
