@@ -619,14 +619,18 @@ __global__ void __launch_bounds__(128, SF_GEN_BLOCKS_PER_SM) k_contacts_gen(Cont
 }
 // The same with the scene's bucket table in shared memory: read from memory, the 27 buckets' bounds and their entries,
 // mostly bricks of elsewhere that share the hash, were some 50 L2 sectors a brick, which is what bounded the pass. A block
-// takes runs of GEN_TAB_RUN consecutive bricks and loads the table of each scene they lie in (bricks are listed scene by
+// takes runs of consecutive bricks and loads the table of each scene they lie in (bricks are listed scene by
 // scene), and a warp 32 of them at a time. What bounds it now is instruction issue (some 2,000 a warp, half the lanes on).
-// Per launch on the 256-scene mix (4.38M bricks) in free fall 989 -> 505 us, at the contact peak 1,642 -> 1,000 us; a world
-// of 12,000 bricks takes 35 us against the other form's 26, 97,000 bricks in one scene 56 against 62.
+// Per launch on the 256-scene mix (4.38M bricks) in free fall 989 -> 505 us, at the contact peak 1,642 -> 1,000 us.
 constexpr int GEN_TAB_T = 1024;
 constexpr size_t GEN_TAB_SMEM = sizeof(BucketTab) + (GEN_TAB_T / 32) * sizeof(WarpQueue);
 constexpr uint32_t GEN_TAB_RUNS = 4;   // runs a block, about
-constexpr uint32_t GEN_TAB_MIN = 256, GEN_TAB_ALL = 65536;   // bricks a scene on average, and in all, from which it is taken
+// Whether n bricks of k scenes take it. It costs a table's load a scene and two and the signatures (5 to 20 us), and gains the
+// more the fuller the buckets are, that is the larger the scenes. Both together, us more (-: less) than the other form with n
+// in all and n / k a scene: 75,000 and 500 +50; 200,000 and 8,000 +24; 300,000 and 2,000 +31, 25,000 +1, 50,000 -6; 700,000 and
+// 8,000 +18, 17,000 +1, 25,000 -15; 1.0M and 4,000 +12, 8,000 -2, 17,000 -27; 1.5M and 2,000 +48, 4,000 -16, 17,000 -72; 4.4M
+// and 4,000 -234, 17,000 -339. Awake bricks of a sparse step count alike (0.57M in 20 scenes +13, 1.3M in 128 -42).
+static bool gen_table(uint64_t n, uint64_t k) { return n * n >= 12500000000ull * k || (n >= 1250000 && n >= 4096 * k); }
 __global__ void __launch_bounds__(GEN_TAB_T) k_contacts_gen_tab(ContactArgs A, uint32_t run, uint32_t K, const uint4 *seg,
                                                                 const uint32_t *awk_pos, uint32_t nd_act, uint32_t *runs) {
     extern __shared__ __align__(16) unsigned char s_tab[];
@@ -2828,8 +2832,8 @@ static sf_status substep(sf_world *w, float h) {
     }
     // the hash table (counting sort into the buckets; see k_hash_count)
     SF_CUDA(cudaMemsetAsync(S->bstart.p, 0, nbk * 4, s));
-    // (a scene's table is loaded whole, 192 KB: see k_contacts_gen_tab for both forms' times)
-    const bool tab = nd >= GEN_TAB_ALL && (uint64_t)nd >= (uint64_t)S->act.size() * GEN_TAB_MIN;
+    // (the awake bricks of a sparse step are counted later: about the last substep's)
+    const bool tab = gen_table(sparse ? std::min(nd, S->n_awk) : nd, S->act.size());
     if (tab) SF_CUDA(cudaMemsetAsync(S->bsig.p, 0, nbk * 2, s));
     k_hash_count<<<grid_for(nd, 256), 256, 0, s>>>(nd, klist, w->k_body.p, w->b_scene.p, S->scene_act.p,
                                                    sparse ? S->scene_awake.p : nullptr, S->scene_bricks.p, w->b_alive.p,
@@ -2872,7 +2876,7 @@ static sf_status substep(sf_world *w, float h) {
         }
     }
     if (g0) cudaEventRecord(g0, s);
-    if (tab && n_awk >= GEN_TAB_ALL) {
+    if (tab && gen_table(n_awk, S->act.size())) {
         // runs taken in turn, about GEN_TAB_RUNS a block (an even load without many table loads)
         const uint32_t run = std::max<uint32_t>(GEN_TAB_T, (n_awk / (GEN_TAB_RUNS * w->sms) + 31) / 32 * 32);
         SF_CUDA(cudaMemsetAsync(S->dev.p + DV_RUN, 0, 4, s));
