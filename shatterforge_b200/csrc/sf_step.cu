@@ -126,6 +126,7 @@ struct StepState {
     std::vector<uint32_t> sub_nc;
     double ph_ms[SF_PHASES] = {};
     uint64_t ph_substeps = 0, solve_contact_iters = 0, solve_launches = 0;
+    DBuf<unsigned long long> kept_sum;   // contacts that small substeps' reductions kept (the host never learns each count)
     // contact generation alone: an event pair per launch, folded in with the phases
     std::vector<cudaEvent_t> gen_ev;
     size_t gen_used = 0;
@@ -1367,6 +1368,7 @@ struct SmallArgs {
     uint32_t *perm, *man_a, *man_b, *man_ca, *man_cb, *man_start, *man_count, *man_prio, *man_color;
     uint32_t *bm_count, *masks;                     // per active body, set up here for those that need them
     uint32_t *col_start, *col_list, *jds_off, *dev, *err;
+    unsigned long long *kept_sum;                   // (null without a reduction)
 };
 
 // exclusive sum over the block's threads; *total gets the whole
@@ -1827,6 +1829,7 @@ __global__ void __launch_bounds__(SMALL_T) k_small_build(SmallArgs A) {
         A.dev[DV_COLORS] = ncol;
         A.dev[DV_ROUNDS] = rounds;
         A.dev[DV_KEPT] = nc;
+        if (A.kept_sum) *A.kept_sum += nc;
     }
 }
 
@@ -2614,7 +2617,8 @@ sf_status step_create(sf_world *w) {
     SF_CUDA(cudaMallocHost((void **)&S->h_live_pin, nsc));
     S->live.assign(w->n_scenes, 1);   // every scene steps until a step shows it asleep
     S->act_brick_base.assign(w->n_scenes, NONE);
-    SF_CUDA(S->dev.alloc(DV_N));
+    SF_CUDA(S->dev.alloc(DV_N)); SF_CUDA(S->kept_sum.alloc(1));
+    SF_CUDA(cudaMemsetAsync(S->kept_sum.p, 0, S->kept_sum.bytes(), s));
     SF_CUDA(cudaMemsetAsync(S->dev.p, 0, S->dev.bytes(), s));
     SF_CUDA(cudaMallocHost((void **)&S->h_dev, DV_N * sizeof(uint32_t)));
     std::vector<uint32_t> off(nb);
@@ -2941,6 +2945,7 @@ static sf_status substep(sf_world *w, float h) {
         B.man_start = S->man_start.p; B.man_count = S->man_count.p; B.man_prio = S->man_prio.p; B.man_color = S->man_color.p;
         B.bm_count = S->bm_count.p; B.masks = S->masks.p; B.col_start = S->col_start.p;
         B.col_list = S->col_list.p; B.jds_off = S->jds_off.p; B.dev = S->dev.p; B.err = w->err.p;
+        B.kept_sum = w->P.reduce && w->P.iterations ? S->kept_sum.p : nullptr;
         prof_mark(w);
         k_small_build<<<1, SMALL_T, SMALL_SMEM, s>>>(B);
         L++;
@@ -3135,7 +3140,7 @@ static sf_status substep(sf_world *w, float h) {
         }
         L++;
         S->solve_launches++;
-        S->solve_contact_iters += (uint64_t)ncm * w->P.iterations;
+        if (!(small && w->P.reduce)) S->solve_contact_iters += (uint64_t)ncm * w->P.iterations;
     }
     if (w->P.warm_start) {
         // the table the next substep reads: every solved contact's impulses under its key
@@ -3325,7 +3330,10 @@ sf_status sf_read_profile(sf_world *w, sf_profile *out) {
     for (int p = 0; p < SF_PHASES; p++) out->ms[p] = S->ph_ms[p];
     out->substeps = S->ph_substeps;
     out->solve_launches = S->solve_launches;
-    out->solve_contact_iters = S->solve_contact_iters;
+    unsigned long long kept = 0;
+    SF_CUDA(cudaMemcpyAsync(&kept, S->kept_sum.p, sizeof kept, cudaMemcpyDeviceToHost, w->stream));
+    SF_CUDA(cudaStreamSynchronize(w->stream));
+    out->solve_contact_iters = S->solve_contact_iters + kept * w->P.iterations;
     uint64_t sum = 0;
     for (uint32_t n : S->sub_nc) sum += n;
     out->contacts_sum = sum;
@@ -3338,6 +3346,7 @@ sf_status sf_read_profile(sf_world *w, sf_profile *out) {
 sf_status sf_reset_profile(sf_world *w) {
     if (!w) return SF_ERR_ARG;
     StepState *S = w->step;
+    SF_CUDA(cudaMemsetAsync(S->kept_sum.p, 0, S->kept_sum.bytes(), w->stream));
     for (int p = 0; p < SF_PHASES; p++) S->ph_ms[p] = 0.0;
     S->ph_substeps = 0; S->solve_launches = 0; S->solve_contact_iters = 0; S->sub_nc.clear(); S->ev_used = 0;
     S->gen_ms = 0.0; S->gen_bricks = 0; S->gen_used = 0;
