@@ -38,12 +38,19 @@ struct SorParams { double omega, tol; uint32_t max_sweeps, use_cap; };
 constexpr int SOR_CL = 8;                        // blocks of a structure's cluster, or SOR_CL_WIDE for large ones
 constexpr int SOR_CL_WIDE = 16;                  // a non-portable cluster size: structures of SOR_CL_WIDE_MIN bricks
 constexpr uint32_t SOR_CL_WIDE_MIN = 20000;
-constexpr int SOR_FORMS = 7;
+// A form serves the structures whose blocks have at most T x C cells of one parity. Fewer threads have shorter barriers and
+// reductions, and let more clusters of small structures run side by side (8, 4 and 2 blocks an SM for the first three); more
+// cells a thread make its chain longer. us a sweep, of the forms that hold a block's cells of one parity: 69 cells 0.60 in 96 x 1,
+// 0.61 in 224 x 1; 191 0.68 in 224 x 1, 0.68 in 480 x 1, 0.82 in 480 x 2; 286 0.76 in 480 x 1, 0.88 in 480 x 2; 585 0.99 in 480 x
+// 2, 1.06 in 608 x 2, 1.28 in 480 x 3; 1,136 1.54 in 608 x 2, 1.84 in 640 x 2 (fewer registers a thread), 1.87 in 480 x 3; 1,420
+// 1.98 in 480 x 3, 2.86 in 992 x 3. 900 structures of 64 bricks 5.5 in 32 x 1, 9.0 in 96 x 1, 18.8 in 224 x 1, and 6 sweeps of
+// them, which the set-up of a cluster bounds, 114, 189, 372 us (288 with all clusters of 256 threads before the halo copies).
 // The last two spill a part of what a cell keeps, and take more threads to hide it: with 16 blocks, us a sweep, a solid of 40^3
 // bricks (2,000 cells of one parity a block) 5.3 in 992 x 3 (480 x 5: 4.7, 736 x 4: 5.5), 125 x 4 x 125 (1,954) 4.1 (4.7, 4.6),
 // a trellis of 65,000 (3,144) 5.7 in 992 x 4 (480 x 9: 7.5, 736 x 6: 7.0, 992 x 5: 6.4).
-constexpr int SOR_FORM_T[SOR_FORMS] = {224, 480, 480, 608, 480, 992, 992};
-constexpr int SOR_FORM_C[SOR_FORMS] = {1, 1, 2, 2, 3, 3, 4};
+constexpr int SOR_FORMS = 9, SOR_SMALL = 2;      // the first SOR_SMALL in solves of many such (solve_impl)
+constexpr int SOR_FORM_T[SOR_FORMS] = {32, 96, 224, 480, 480, 608, 480, 992, 992};
+constexpr int SOR_FORM_C[SOR_FORMS] = {1, 1, 1, 1, 2, 2, 3, 3, 4};
 constexpr uint32_t SOR_CL_CAP = 3968;            // cells of one parity a block takes at most (the last form's T x C)
 constexpr int SOR_NCLS = 2 * SOR_FORMS;          // launch classes: a form, with 16 or 8 blocks
 
@@ -403,7 +410,7 @@ struct SorClusterArgs {
     const uint32_t *ccode;
     const int32_t *csid;
     uint32_t stride;                             // potentials of one buffer: the largest block's cells and halo, and one
-    uint32_t push_max, ps_max;                   // shared-memory entries of the push tables
+    uint32_t push_max;                           // shared-memory entries of the push table (the starts follow it)
     const SorParams *prm;
     uint32_t *sweeps;
     double *resid;
@@ -487,7 +494,7 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
 }
 
 template <int T, int C>
-__global__ void __launch_bounds__(T + 32, T < 256 ? 2 : 1) k_sor_cluster(SorClusterArgs A) {
+__global__ void __launch_bounds__(T + 32, T <= 32 ? 8 : T <= 96 ? 4 : T < 256 ? 2 : 1) k_sor_cluster(SorClusterArgs A) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char sm[];
@@ -1168,7 +1175,9 @@ static SorKernel sor_cluster_kernel(int form) {
         case 3: return k_sor_cluster<SOR_FORM_T[3], SOR_FORM_C[3]>;
         case 4: return k_sor_cluster<SOR_FORM_T[4], SOR_FORM_C[4]>;
         case 5: return k_sor_cluster<SOR_FORM_T[5], SOR_FORM_C[5]>;
-        default: return k_sor_cluster<SOR_FORM_T[6], SOR_FORM_C[6]>;
+        case 6: return k_sor_cluster<SOR_FORM_T[6], SOR_FORM_C[6]>;
+        case 7: return k_sor_cluster<SOR_FORM_T[7], SOR_FORM_C[7]>;
+        default: return k_sor_cluster<SOR_FORM_T[8], SOR_FORM_C[8]>;
     }
 }
 static size_t sor_cluster_smem(uint32_t stride, uint32_t push, uint32_t ps) { return (size_t)stride * 16 + (size_t)push * 8 + (size_t)ps * 4; }
@@ -1483,7 +1492,12 @@ static sf_status solve_impl(sf_world *w, int32_t structure, const int32_t *ids, 
         auto expect = [&](uint32_t q) -> double {
             return (st->h_last_sweeps[q] ? (double)st->h_last_sweeps[q] : st->h_guess[q]) * (600.0 + st->h_cl[q].half);
         };
-        for (uint32_t q : req) by_cls[st->h_cl[q].cls].push_back(q);
+        // The forms of small blocks pay where the next one's clusters (two blocks an SM) would not all run at once. Beside large
+        // structures they took SMs that those had to wait for (the 37-building lattice 51 ms, 41.5 without).
+        uint32_t small = 0;
+        for (uint32_t q : req) small += st->h_cl[q].cls < 2 * (uint32_t)SOR_SMALL ? 1 : 0;
+        const uint32_t least = small == req.size() && small * (uint32_t)SOR_CL > 2u * w->sms ? 0u : 2 * (uint32_t)SOR_SMALL;
+        for (uint32_t q : req) by_cls[std::max(st->h_cl[q].cls, least)].push_back(q);
         for (int c = 0; c < SOR_NCLS; c++) {
             std::stable_sort(by_cls[c].begin(), by_cls[c].end(), [&](uint32_t a, uint32_t b) { return expect(a) > expect(b); });
             uint32_t *sh = shape + 4 * c;
@@ -1537,7 +1551,7 @@ static sf_status solve_impl(sf_world *w, int32_t structure, const int32_t *ids, 
             X.cap = st->cap.p;
             X.list = st->cl_list.p + first; X.blk = st->cl_blk.p; X.cpos = st->cl_cpos.p; X.hpos = st->cl_hpos.p;
             X.hface = st->cl_hface.p; X.nbr = st->cl_nbr.p; X.ps = st->cl_ps.p; X.push = st->cl_push.p; X.cphi = st->cphi.p; X.crhs = st->crhs.p;
-            X.ccode = st->ccode.p; X.csid = st->csid.p; X.stride = sh[1]; X.push_max = sh[2]; X.ps_max = sh[3];
+            X.ccode = st->ccode.p; X.csid = st->csid.p; X.stride = sh[1]; X.push_max = sh[2];
             X.prm = st->prm.p; X.sweeps = st->sweeps.p; X.resid = st->resid.p; X.err = w->err.p;
             const unsigned ncl = (c & 1) ? (unsigned)SOR_CL_WIDE : (unsigned)SOR_CL;
             cattr[c][0].id = cudaLaunchAttributeClusterDimension;
