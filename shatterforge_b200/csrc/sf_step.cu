@@ -2016,11 +2016,12 @@ __global__ void __launch_bounds__(SOLVE_BLOCK) k_solve(SolveArgs A) {
 // of colour c in block (p + c) % NB, so that colours of one manifold, a large body's, fill all the blocks) and the places of
 // both. What bounds a colour pass there is the chain of its longest manifold, up to 32 contacts of some 300 dependent-issue
 // operations; read from L2 a contact took 780 to 930 cycles, the latency of its six words.
-// Solve of 8 iterations, against one block (or warp) that read everything through L1: 1,300 contacts 140 -> 107 us (alone;
-// 114 on the cluster), 2,980 198 -> 143 us, 3,600 242 -> 133 us, 7,580 288 -> 147 us. A contact then took 590 cycles, about
-// its instructions at one every two cycles of the one warp that runs the chain. One body on the ground, whose colours are a
-// manifold each, ms: 576 contacts 1.33 -> 1.14 (470 cycles a contact without the second body's side), 2,500 6.83 -> 4.23, 7,200
-// 22.4 -> 12.2; with places for 64 colours only and every such colour in block 0, these took 1.50, 8.9 and 25.4.
+// Solve of 8 iterations, against one block (or warp) that read everything through L1, us: 1,240 contacts (alone) 143 -> 96, 2,980
+// 236 -> 138, 3,850 with reduction and warm start 317 -> 167, 6,760 299 -> 139. One body on the ground, whose colours are a manifold
+// each, ms: 576 contacts 1.33 -> 1.02, 2,500 6.83 -> 3.90, 7,200 22.4 -> 11.2; with places for 64 colours only and every such
+// colour in block 0, these took 1.50, 8.9 and 25.4. A contact takes some 420 cycles without the second body's side, about its
+// instructions at one every two cycles of the one warp that runs the chain. (One block an SM is stated, as the compiler else
+// spares registers for four: 3,850 contacts 188 us.)
 constexpr int SOLVE_TEAM_BLOCKS = 16, SOLVE_TEAM_T = 128, SOLVE_TEAM_T1 = 256;   // threads a block of the cluster / alone
 constexpr uint32_t SOLVE_TEAM_MAX = 8192;          // contacts
 constexpr uint32_t SMALL_SUBSTEP_CONTACTS = 1024;  // contacts up to which the colouring runs on one block
@@ -2046,7 +2047,7 @@ __device__ __forceinline__ void cp_async16(float4 *to, const float4 *from) {
 // L1, a cluster through L2 (its barriers order them). A step of 80,000 bodies of which 100 lie in a heap (180 contacts) takes 0.61
 // ms so; with the kernels of large substeps it took 1.24, with the former one-block solve and separate launches 1.03.
 template <int NB, int T, bool NEAR>
-__global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *nc_p, uint32_t K, uint32_t slots, uint32_t max_rows) {
+__global__ void __launch_bounds__(T, 1) k_solve_team(SolveArgs A, const uint32_t *nc_p, uint32_t K, uint32_t slots, uint32_t max_rows) {
     static_assert((NB & (NB - 1)) == 0, "a power of two");
     extern __shared__ float4 sv[];                 // velocity, spin of bodies rank, rank + NB, ...; the contacts; the places
     __shared__ uint32_t s_base[NB];                // shared::cluster address of every block's velocities
@@ -2189,14 +2190,12 @@ __global__ void __launch_bounds__(T) k_solve_team(SolveArgs A, const uint32_t *n
                         x.j = sc[5 * slots + q];
                         return x;
                     };
-                    uint32_t at = loc[0] + lp;
-                    Contact y = get(at);
+                    Contact y = get(loc[0] + lp);
                     for (uint32_t k = 0; k < P.cnt; k++) {
                         const Contact x = y;
-                        const uint32_t own = at;
-                        if (k + 1 < P.cnt) { at = loc[k + 1] + lp; y = get(at); }
+                        if (k + 1 < P.cnt) y = get(loc[k + 1] + lp);
                         if (warm) warm_contact(P, x);
-                        else sc[5 * slots + own] = solve_contact<SIDES>(P, x);
+                        else sc[5 * slots + loc[k] + lp] = solve_contact<SIDES>(P, x);
                     }
                 } else {
                     const uint32_t *off = A.jds_off + c0 * JDS_K;
