@@ -1138,17 +1138,18 @@ extern "C" sf_status sf_box_world_create(const float *boxes, const uint32_t *sce
             if (cudaOccupancyMaxActiveClusters(&ncl, k_box_step<BX_CL_THREADS, BX_CL>, &c) != cudaSuccess) { ncl = 0; cudaGetLastError(); }
             w->cluster_ok = ncl > 0;
         }
-        // A cluster's barriers cost what a block's longer loops do at some 1,000 boxes. Measured a pass of two steps of 12 (4)
-        // sub-steps, block against cluster: one scene of 700 boxes 2.3, 2.4 ms; 1,000 2.9, 2.7 (2.6, 1.8); 2,000 5.0, 3.0 (3.8,
-        // 1.7); 4,000 10.4, 3.9; but eight of 2,000, one more than fit at once, 5.5, 6.5. A world of fewer boxes in some
-        // scene keeps its one-block launch, which would run after the clusters.
+        // A cluster's barriers cost what a block's longer loops do at some 1,000 boxes. Two steps of 12 (4) sub-steps, ms, block
+        // against cluster: one scene of 500 boxes 1.84, 2.24 (1.14, 1.20); 700 2.14, 2.24 (1.75, 1.39); 1,000 2.89, 2.68 (2.08,
+        // 1.51); 2,000 5.19, 3.26 (3.70, 1.75); 4,000 10.3, 4.1 (7.0, 2.0); seven of 2,000 5.33, 3.39 (3.77, 1.77); but eight of
+        // 2,000, one more than fit at once, 5.37, 6.64 (3.78, 3.41). A world of fewer boxes in some scene keeps its one-block
+        // launch, which would run after the clusters.
         const uint32_t line = least > BX_MID && n_scenes <= (uint32_t)ncl ? BX_MID : BX_BIG;
         std::vector<uint32_t> big, small;
         for (uint32_t s = 0; s < n_scenes; s++) (w->nn[s] > line ? big : small).push_back(s);
         w->n_big = (uint32_t)big.size(); w->n_small = (uint32_t)small.size();
-        // One block an SM is enough for the scenes: 512 threads each, not two blocks of 256. Measured a pass of two steps:
-        // 148 scenes of 2,000 boxes 11.3 against 15.1 ms, one of 2,000 6.9 against 9.9, but 300 of 300 5.7 against 4.5, and
-        // under 256 boxes a scene nothing (148 of 100: 1.43 against 1.35 ms), as 256 threads reach every box in one go.
+        // One block an SM is enough for the scenes: 512 threads each, not two blocks of 256. Two steps of 12 sub-steps, ms: 148
+        // scenes of 2,000 boxes 8.5 against 11.6, of 300 1.38, 1.52; one of 2,000 5.2, 7.0, of 300 1.18, 1.32; but 200 of 300 2.46,
+        // 1.83, and under 256 boxes a scene next to nothing (148 of 100 0.60, 0.61), as 256 threads reach every box in one go.
         uint64_t sn = 0;
         for (uint32_t s : small) sn += w->nn[s];
         int dev = 0, sms = 0;

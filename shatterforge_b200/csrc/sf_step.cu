@@ -621,7 +621,8 @@ __global__ void __launch_bounds__(128, SF_GEN_BLOCKS_PER_SM) k_contacts_gen(Cont
 // The same with the scene's bucket table in shared memory: read from memory, the 27 buckets' bounds and their entries,
 // mostly bricks of elsewhere that share the hash, were some 50 L2 sectors a brick, which is what bounded the pass. A block
 // takes runs of consecutive bricks and loads the table of each scene they lie in (bricks are listed scene by
-// scene), and a warp 32 of them at a time. What bounds it now is instruction issue (some 2,000 a warp, half the lanes on).
+// scene), and a warp 32 of them at a time. What bounds it now is the L2 latency of the entries and positions behind the table
+// with one block an SM (issue 43 % busy, long-scoreboard 7.2 and barrier 4.2 stalls an issue, of some 2,000 instructions a warp).
 // Per launch on the 256-scene mix (4.38M bricks) in free fall 989 -> 505 us, at the contact peak 1,642 -> 1,000 us.
 constexpr int GEN_TAB_T = 1024;
 constexpr size_t GEN_TAB_SMEM = sizeof(BucketTab) + (GEN_TAB_T / 32) * sizeof(WarpQueue);
@@ -1343,9 +1344,9 @@ __global__ void k_col_verify(const uint32_t *nm_p, const uint32_t *man_a, const 
 // The manifolds of a substep of at most SMALL_MAX contacts, their colours and the contact layout, by one block: the
 // contacts sorted by pair, reduced, cut into chunks, coloured and listed as the kernels above do it (the same manifolds,
 // colours and rounds; only the order inside a list's bucket is free). Those are some forty-five launches, which is what
-// bounds them on few contacts; the one block is bound by the latency of its phases (2 to 4 us each, a colouring round 2).
-// Against those launches: 1,300 contacts (12 rounds) 276 -> 59 us, 2,980 (13) 332 -> 82, 3,450 with reduction 264 -> 58,
-// 7,580 (4) 230 -> 56 us.
+// bounds them on few contacts; the one block is bound by the latency of its phases (2 to 4 us each, a colouring round 1) and of
+// its instructions, which each warp meets once (no-instruction stalls lead in a capture). Against those launches, us: 1,240
+// contacts 262 -> 37, 2,980 360 -> 56, 3,850 with reduction 278 -> 66, 6,760 221 -> 52.
 constexpr int SMALL_T = 1024, SMALL_ITEMS = 8;
 constexpr uint32_t SMALL_MAX = SMALL_T * SMALL_ITEMS;
 constexpr uint32_t MASK_DEG = 32;      // manifolds of a body above which its colours are kept as a mask
