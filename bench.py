@@ -42,15 +42,16 @@ UNIT = "body-steps/s"
 DT = 1.0 / 60.0
 ITERS = 8
 SOLVE_BYTES_PER_CONTACT_ITER = 184     # contact 64 + impulse r/w 24 + both bodies' v, w r/w 96
-# DRAM bytes (read + write) per contact-iteration of k_solve, from one ncu capture at the peak of contacts on the
-# half-size mix: 722.7 MB for that launch / (≈847,700 contacts, from the same substep's k_prep grid, x 8 iterations);
-# the roofline's `traffic` scales it to this run's average launch
-SOLVE_DRAM_BYTES_PER_CONTACT_ITER = 106.6
+# DRAM bytes (read + write) per contact-iteration of k_solve on the 256-scene mix, from one-pass ncu captures of launches of
+# 1.885M contacts (step 110: 2,336 MB, 8 iterations) and of 23,700 (step 15, whose contacts stay in L2: 8.6 MB); the
+# roofline's `traffic` scales them to this run's average launch
+SOLVE_DRAM_BYTES_PER_CONTACT_ITER = (155.0, 45.6)
+SOLVE_RESIDENT_CONTACTS = 1_000_000    # contacts a launch up to which the latter holds: their 126 B each fit the 126 MB L2
 GEN_BYTES_PER_BRICK = 40               # local offset 12 + body id 4 read, world position 12 written and re-read
 GEN_BYTES_PER_CONTACT = 64             # one contact's setup written
-# DRAM bytes (read + write) of k_contacts_gen per algorithmic byte, from the ncu capture in free fall on the half-size
-# mix (the benchmark window's regime): 77.2 MB against 40 B x 1.11M bricks + 64 B x ~4,000 contacts
-GEN_DRAM_PER_ALGORITHMIC_BYTE = 1.73
+# DRAM bytes (read + write) of k_contacts_gen_tab per algorithmic byte, from a one-pass ncu capture on the 256-scene mix in
+# free fall (step 15, the benchmark window's regime): 278.8 MB against 40 B x 4.38M bricks + 64 B x 23,700 contacts
+GEN_DRAM_PER_ALGORITHMIC_BYTE = 1.58
 SOR_BYTES_PER_BRICK_SWEEP = 24         # grid path: f64 potential r/w 16 + rhs 4 + link word 4
 SOR_CLUSTER_BYTES_PER_BRICK = 52       # cluster path, once per solve: staging reads (phi 8, rhs 4, code 4, sid 4,
                                        # place 4, neighbours 12) + the potential written back 8 + gather 8
@@ -772,14 +773,15 @@ def our_arm(args, rank, world, local, pg):
     solve_ms = phase_ms["solve"]
     solve_bytes = SOLVE_BYTES_PER_CONTACT_ITER * prof["solve_contact_iters"]
     nsl = max(prof["solve_launches"], 1)
+    solve_dram = SOLVE_DRAM_BYTES_PER_CONTACT_ITER[prof["solve_contact_iters"] / nsl / ITERS <= SOLVE_RESIDENT_CONTACTS]
     roof_solve = {"kernel": "k_solve (coloured sequential-impulse solve)", "bound": "hbm",
                   "achieved": solve_bytes / max(solve_ms * 1e-3, 1e-12) / 1e9, "peak": hbm, "peak_source": peak_source,
-                  "unit": "GB/s", "traffic": SOLVE_DRAM_BYTES_PER_CONTACT_ITER * prof["solve_contact_iters"] / nsl,
+                  "unit": "GB/s", "traffic": solve_dram * prof["solve_contact_iters"] / nsl,
                   "bytes_per_launch": solve_bytes / nsl, "ms_per_launch": solve_ms / nsl, "launches": int(prof["solve_launches"]),
                   "unit_bytes": f"{SOLVE_BYTES_PER_CONTACT_ITER} B per contact-iteration"}
     roof_solve["frac"] = roof_solve["achieved"] / hbm
     gen_bytes = GEN_BYTES_PER_BRICK * prof["gen_bricks"] + GEN_BYTES_PER_CONTACT * prof["contacts_sum"]
-    roof_gen = {"kernel": "k_contacts_gen (broad and narrow phase, one thread per awake brick)", "bound": "hbm",
+    roof_gen = {"kernel": "k_contacts_gen_tab (broad and narrow phase, bucket tables in shared memory; k_contacts_gen in smaller worlds)", "bound": "hbm",
                 "achieved": gen_bytes / max(prof["gen_ms"] * 1e-3, 1e-12) / 1e9, "peak": hbm, "peak_source": peak_source,
                 "unit": "GB/s", "traffic": GEN_DRAM_PER_ALGORITHMIC_BYTE * gen_bytes / launches,
                 "bytes_per_launch": gen_bytes / launches, "ms_per_launch": prof["gen_ms"] / launches, "launches": launches,
@@ -848,7 +850,7 @@ def our_arm(args, rank, world, local, pg):
         cluster = int(ws.stats().cluster_solves) > 0
         if cluster:
             # cells stay in shared memory for the whole solve: HBM is read and written once per solve, and a sweep
-            # costs two cluster barriers and two dependent f64 cell updates, so the solve takes the critical
+            # costs two halo waits with a block barrier each and two dependent f64 cell updates, so the solve takes the critical
             # structure's sweep count times its time per sweep
             roof = {"bound": "sync", "unit": "us per sweep of the critical structure",
                     "achieved": s_ms * 1e3 / max(rep.max_sweeps_done, 1),
