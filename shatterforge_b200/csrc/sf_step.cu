@@ -1964,17 +1964,23 @@ __device__ __forceinline__ void warm_contact(Pair &P, const Contact &c) {
 }
 
 // manifold i of the colour lists, the p-th of its colour
-__device__ __forceinline__ void solve_manifold(const SolveArgs &A, uint32_t i, uint32_t p, const uint32_t *off, bool warm) {
-    Pair P = load_pair(A, i);
-    load_vel(A, P);
+template <Sides SIDES>
+__device__ __forceinline__ void solve_contacts(const SolveArgs &A, Pair &P, uint32_t p, const uint32_t *off, bool warm) {
     // the next contact's data is loaded while the current one is solved (the chain through the bodies is serial)
     Contact nx = load_contact<false>(A, off[0] + p);
     for (uint32_t k = 0; k < P.cnt; k++) {
         const Contact c = nx;
         if (k + 1 < P.cnt) nx = load_contact<false>(A, off[k + 1] + p);
         if (warm) warm_contact(P, c);
-        else A.S_j[off[k] + p] = solve_contact<BRANCH>(P, c);
+        else A.S_j[off[k] + p] = solve_contact<SIDES>(P, c);
     }
+}
+__device__ __forceinline__ void solve_manifold(const SolveArgs &A, uint32_t i, uint32_t p, const uint32_t *off, bool warm) {
+    Pair P = load_pair(A, i);
+    load_vel(A, P);
+    // lanes whose manifolds are all against the ground or static bodies leave the second side out
+    if (__any_sync(__activemask(), P.hasb)) solve_contacts<BRANCH>(A, P, p, off, warm);
+    else solve_contacts<NO_SECOND>(A, P, p, off, warm);
     store_vel(A, P);
 }
 

@@ -1,4 +1,4 @@
-"""The solve of small substeps with many colours, against the oracle bit for bit: a slab on the ground under a layer of single
+"""The solve of substeps with many colours, against the oracle bit for bit: a slab on the ground under a layer of single
 bricks, with chunks of 1, 16 and 32 contacts (the last has more rows of places than are kept in shared memory), alone and on a
 cluster, with and without a warm start."""
 import numpy as np
@@ -10,12 +10,12 @@ pytestmark = pytest.mark.gpu
 DT, IT = 1.0 / 60.0, 3
 
 
-def laden_slab(w):
-    """A slab of w x w bricks on the ground and a single brick on each of its bricks."""
+def laden_slab(w, every=1):
+    """A slab of w x w bricks on the ground and a single brick on every `every`-th of its bricks."""
     a = S.body_blocks(1, w, w, 1)
-    n = w * w
+    k = np.arange(0, w * w, every)
+    n = len(k)
     f, x, m, p = S.loose_debris(n, 1)
-    k = np.arange(n)
     p[:, 0:3] = np.stack([0.5 * (k % w), np.full(n, 0.52), 0.5 * (k // w)], 1)
     return S.Scene(a.static_xyz, a.static_mat, a.static_sid, a.static_infill,
                    np.concatenate([a.body_first, a.body_first[-1] + f[1:]]).astype(np.uint32),
@@ -39,6 +39,24 @@ def test_many_colours_equal_oracle(sf, oracle, w, chunk, warm, colours):
             np.testing.assert_array_equal(x, y)
         np.testing.assert_array_equal(g.manifolds(0), ow.manifolds())
     assert most >= colours
+    g.close()
+
+
+@pytest.mark.parametrize("warm", [0, 1])
+def test_a_large_substep_of_many_colours_equals_oracle(sf, oracle, warm):
+    """8,464 contacts of the slab with the ground and some of its bricks' with single ones: warps of k_solve with and without
+    second bodies."""
+    sc = laden_slab(46, 13)
+    g = sf.World(sc, iterations=IT, max_colors=1024, warm_start=warm)
+    ow = oracle.OracleWorld(sc)
+    most = 0
+    for _ in range(2):
+        most = max(most, g.step(DT).contacts)
+        ow.step(DT, iterations=IT, order=oracle.ORDER_COLOR, warm=warm)
+        for x, y in zip(g.bodies(), ow.bodies()):
+            np.testing.assert_array_equal(x, y)
+        np.testing.assert_array_equal(g.manifolds(0), ow.manifolds())
+    assert most > 8192
     g.close()
 
 
